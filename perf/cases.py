@@ -529,7 +529,7 @@ class Handle:
             ctypes.byref(self.h)))
 
     def __del__(self):
-        if self.h:
+        if self.h and _lib is not None:  # None while the interpreter exits
             _lib.lib.pmg_problem_destroy(self.h)
 
 
