@@ -44,6 +44,7 @@
 #include <cuda.h>
 
 #include "gs27_tiled.cuh"
+#include "mbar.cuh"
 
 namespace pmg {
 
@@ -108,56 +109,11 @@ __global__ void coef_split_kernel(Dims d, CoefSplit cs, Op14<float> A,
   }
 }
 
-// mbarrier polls before the stage counts as lost: about 0.1 s, some 10^4
-// times the longest real wait
-constexpr long kTmaMaxPolls = 1L << 20;
-
 // Tensor maps of the two iterate buffers in the roles of the launch.
 struct alignas(64) Gs27TmaMaps {
   CUtensorMap own, nb;
 };
 
-__device__ __forceinline__ unsigned smem_addr(const void *p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(
-                   smem_addr(bar)),
-               "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar,
-                                               unsigned bytes) {
-  asm volatile(
-      "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
-          smem_addr(bar)),
-      "r"(bytes)
-      : "memory");
-}
-// true once the phase with this parity has completed
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar,
-                                              unsigned parity) {
-  unsigned done;
-  asm volatile("{\n"
-               ".reg .pred p;\n"
-               "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-               "selp.u32 %0, 1, 0, p;\n"
-               "}\n"
-               : "=r"(done)
-               : "r"(smem_addr(bar)), "r"(parity)
-               : "memory");
-  return done != 0;
-}
-// bounded wait: false if the phase did not complete within kTmaMaxPolls
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
-  for (long n = 0; n < kTmaMaxPolls; ++n) {
-    if (mbar_try_wait(bar, parity))
-      return true;
-    if (n > 64)
-      __nanosleep(64);
-  }
-  return false;
-}
 // one box of a 3-D tensor map into shared memory, completing on bar
 __device__ __forceinline__ void tma_load_3d(float *dst, const CUtensorMap *map,
                                             int x, int y, int z,
@@ -180,9 +136,6 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src,
 
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 }
 
 // Sub-colour step S (points (i, j) with i % 2 = S & 1, j % 2 = S >> 1) with

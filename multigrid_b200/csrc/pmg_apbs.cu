@@ -7,6 +7,10 @@
 // ac + s*nx*ny*nz, in the order oC oE oN uC (7-point, 4 columns) or oC oE oN
 // uC oNE oNW uE uW uN uS uNE uNW uSE uSW (27-point, 14 columns); ipc[10]
 // (the reference's VAT(ipc, 11)) is 7 or 27.
+#include <algorithm>
+#include <type_traits>
+
+#include "cg_cluster.cuh"
 #include "launch.cuh"
 #include "reduce_kernels.cuh"
 #include "pmg_b200.h"
@@ -140,6 +144,30 @@ struct CghsScratch {
   }
 };
 
+// Vcghs on a grid that fits on chip (cg_cluster.cuh): one launch, the count
+// left on the device in *it (a caller that does not need it does not wait).
+template <int KIND>
+int cghs_on_chip(const Dims &d, const Op14<double> &A, const double *cc,
+                 const double *fc, double *x, double *pv, double *ap,
+                 double *r, int itmax, int *it, double errtol,
+                 cudaStream_t s) {
+  // p's shell reads as zero afterwards, as the general path leaves it
+  PMG_CUDA_TRY(cudaMemsetAsync(pv, 0, sizeof(double) * d.count(), s));
+  CgArgs a{};
+  a.d = d;
+  a.A = A;
+  a.cc = cc;
+  a.rhs = fc;
+  a.x = x;
+  a.r = r;
+  a.p = pv;
+  a.ap = ap;
+  a.errtol = errtol;
+  a.max_iters = itmax;
+  a.status = it;
+  return launch_cg_on_chip<KIND, true>(a, s);
+}
+
 template <int KIND>
 int cghs(const Dims &d, const Op14<double> &A, const double *cc,
          const double *fc, double *x, double *pv, double *ap, double *r,
@@ -147,6 +175,30 @@ int cghs(const Dims &d, const Op14<double> &A, const double *cc,
   *iters = 0;
   if (*iters >= itmax && iresid == 0)
     return PMG_OK;
+  if (cg_cluster_fits(d)) {
+    int *it = nullptr;
+    PMG_CUDA_TRY(scratch_alloc((void **)&it, sizeof(int), s));
+    int rc = cghs_on_chip<KIND>(d, A, cc, fc, x, pv, ap, r, itmax, it,
+                                errtol, s);
+    cudaError_t e = cudaSuccess;
+    if (rc == PMG_OK)
+      e = cudaMemcpyAsync(iters, it, sizeof(int), cudaMemcpyDeviceToHost, s);
+    scratch_free(it, s);
+    if (rc != PMG_OK)
+      return rc;
+    if (e == cudaSuccess)
+      e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+      set_last_error(e, "Vcghs", __FILE__, __LINE__);
+      return PMG_ERR_CUDA;
+    }
+    if (*iters < 0) {
+      set_last_message("Vcghs: a message between CTAs did not arrive");
+      *iters = 0;
+      return PMG_ERR_TIMEOUT;
+    }
+    return PMG_OK;
+  }
   const dim3 rg = reduce_grid(d), rb = interior_block();
   const size_t nb = (size_t)rg.x * rg.y * rg.z;
   CghsScratch w(s);
@@ -272,7 +324,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 
 // r = f - A x (Vmresid order) and its L1 norm: the stop test of istop 0/1
 // (mgcsd.cc:467-481).
-template <int KIND>
+template <int KIND, int PL>
 __global__ void __launch_bounds__(kReduceThreads)
     apbs_resid_l1_kernel(Dims d, Op14<double> A, const double *__restrict__ cc,
                          const double *__restrict__ fc,
@@ -281,11 +333,14 @@ __global__ void __launch_bounds__(kReduceThreads)
   __shared__ double sh[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k0 = 2 + blockIdx.z * kReducePlanes;
-  const int k1 = min(k0 + kReducePlanes - 1, d.nz - 1);
+  const int k0 = 2 + blockIdx.z * PL;
   double acc = 0.0;
   if (i <= d.nx - 1 && j <= d.ny - 1)
-    for (int k = k0; k <= k1; ++k) {
+#pragma unroll
+    for (int q = 0; q < PL; ++q) {
+      const int k = k0 + q;
+      if (k > d.nz - 1)
+        break;
       const int p = d.at(i, j, k);
       const double v = resid_at<KIND>(A, cc, fc, x, p, d.sy(), d.sz());
       r[p] = v;
@@ -297,7 +352,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 
 // Hackbusch-Reusken damping of the coarse correction (mgcsd.cc:431-439):
 // w = (x . w0) / (x . A x), A with cc (Vmatvec), over the coarse interior.
-template <int KIND>
+template <int KIND, int PL>
 __global__ void __launch_bounds__(kReduceThreads)
     apbs_damp_kernel(Dims d, Op14<double> A, const double *__restrict__ cc,
                      const double *__restrict__ x,
@@ -306,11 +361,14 @@ __global__ void __launch_bounds__(kReduceThreads)
   __shared__ double sh[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k0 = 2 + blockIdx.z * kReducePlanes;
-  const int k1 = min(k0 + kReducePlanes - 1, d.nz - 1);
+  const int k0 = 2 + blockIdx.z * PL;
   double up = 0.0, lo = 0.0;
   if (i <= d.nx - 1 && j <= d.ny - 1)
-    for (int k = k0; k <= k1; ++k) {
+#pragma unroll
+    for (int q = 0; q < PL; ++q) {
+      const int k = k0 + q;
+      if (k > d.nz - 1)
+        break;
       const int p = d.at(i, j, k);
       up += x[p] * w0[p];
       lo += x[p] * apply_op<KIND>(A, cc, x, p, d.sy(), d.sz());
@@ -535,6 +593,29 @@ struct ApbsLevel {
   (L).a(0), (L).a(1), (L).a(2), (L).a(3), (L).a(4), (L).a(5), (L).a(6),        \
       (L).a(7), (L).a(8), (L).a(9), (L).a(10), (L).a(11), (L).a(12), (L).a(13)
 
+// f with the planes per block of the level's reductions (lambda_planes) as a
+// compile-time constant: the plane loop unrolls, so a thread's loads are in
+// flight together, and small levels launch a block per plane (27-point
+// damping at 33^3 and below: 21 us with eight planes in turn).
+template <class F> void by_planes(const Dims &d, F f) {
+  const int pl = lambda_planes(d);
+  if (pl == 4)
+    f(std::integral_constant<int, 4>{});
+  else if (pl == 2)
+    f(std::integral_constant<int, 2>{});
+  else
+    f(std::integral_constant<int, 1>{});
+}
+
+// blocks of the largest reduction of a driver's levels
+template <class L> size_t reduce_blocks(const L *lv, int nlev) {
+  size_t n = 1;
+  for (int q = 1; q <= nlev; ++q)
+    for (const dim3 g : {reduce_grid(lv[q].d), lambda_grid(lv[q].d)})
+      n = std::max(n, (size_t)g.x * g.y * g.z);
+  return n;
+}
+
 Op14<double> level_op(const ApbsLevel &L) {
   Op14<double> A{};
   for (int s = 0; s < (L.kind == 7 ? 4 : 14); ++s)
@@ -571,7 +652,6 @@ struct ApbsDriver {
   void *block = nullptr; // every level array and work vector
   double *partials = nullptr, *res = nullptr;
   unsigned *ticket = nullptr;
-  dim3 rg0;
 
   explicit ApbsDriver(cudaStream_t st) : s(st) {}
   ~ApbsDriver() {
@@ -612,6 +692,17 @@ struct ApbsDriver {
     return fetch(res, host);
   }
 
+  // Vcghs of a level that fits on chip, queued: nothing in the cycle reads
+  // its iteration count
+  int cg_queued(ApbsLevel &L, const double *f, double *x, double *p,
+                double *ap, double *r, int itmax, double errtol) {
+    int *it = (int *)(ticket + 1);
+    return L.kind == 7 ? cghs_on_chip<7>(L.d, level_op(L), L.cc, f, x, p, ap,
+                                         r, itmax, it, errtol, s)
+                       : cghs_on_chip<27>(L.d, level_op(L), L.cc, f, x, p,
+                                          ap, r, itmax, it, errtol, s);
+  }
+
   // Vsmooth (smoothd.cc:58-87): red-black GS (then the residual into w1
   // when iresid) or the CG with errtol 0 (its residual is w1).
   int smooth(ApbsLevel &L, const double *f, double *x, int nu, int iadjoint,
@@ -619,6 +710,8 @@ struct ApbsDriver {
     const Dims &d = L.d;
     int rc = PMG_OK;
     if (mgsmoo == 4) {
+      if ((nu > 0 || iresid) && cg_cluster_fits(d))
+        return cg_queued(L, f, x, w2, w3, w1, nu, 0.0);
       int it = 0;
       return pmg_Vcghs_d(d.nx, d.ny, d.nz, L.ipc, L.ac, L.cc, f, x, w2, w3,
                          w1, nu, &it, 0.0, iresid, s);
@@ -656,6 +749,8 @@ struct ApbsDriver {
       return faces(C, C.x, nullptr, nullptr, nullptr);
     }
     PMG_CUDA_TRY(cudaMemsetAsync(C.x, 0, sizeof(double) * C.d.count(), s));
+    if (cg_cluster_fits(C.d))
+      return cg_queued(C, f, C.x, w1, w2, w3, 100, epsiln);
     int it = 0;
     return pmg_Vcghs_d(C.d.nx, C.d.ny, C.d.nz, C.ipc, C.ac, C.cc, f, C.x, w1,
                        w2, w3, 100, &it, epsiln, 0, s);
@@ -665,8 +760,11 @@ struct ApbsDriver {
   int stop_norm(int istop, double *tru, double *out) {
     ApbsLevel &F = lv[1];
     if (istop == 0 || istop == 1) {
-      apbs_resid_l1_kernel<7><<<reduce_grid(F.d), interior_block(), 0, s>>>(
-          F.d, level_op(F), F.cc, F.fc, F.x, w1, slot(res));
+      by_planes(F.d, [&](auto pl) {
+        apbs_resid_l1_kernel<7, pl.value>
+            <<<lambda_grid(F.d), interior_block(), 0, s>>>(
+                F.d, level_op(F), F.cc, F.fc, F.x, w1, slot(res));
+      });
       PMG_LAUNCH_CHECK();
       return fetch(res, out);
     }
@@ -727,13 +825,15 @@ struct ApbsDriver {
           rc = coarse(lv[nlev], lv[nlev].w0);
         for (int L = nlev - 1; L >= 1 && rc == PMG_OK; --L) {
           ApbsLevel &F = lv[L], &C = lv[L + 1];
-          if (C.kind == 7)
-            apbs_damp_kernel<7><<<reduce_grid(C.d), interior_block(), 0, s>>>(
-                C.d, level_op(C), C.cc, C.x, C.w0, slot(res), res + 3);
-          else
-            apbs_damp_kernel<27>
-                <<<reduce_grid(C.d), interior_block(), 0, s>>>(
-                    C.d, level_op(C), C.cc, C.x, C.w0, slot(res), res + 3);
+          by_planes(C.d, [&](auto pl) {
+            const dim3 g = lambda_grid(C.d), b = interior_block();
+            if (C.kind == 7)
+              apbs_damp_kernel<7, pl.value><<<g, b, 0, s>>>(
+                  C.d, level_op(C), C.cc, C.x, C.w0, slot(res), res + 3);
+            else
+              apbs_damp_kernel<27, pl.value><<<g, b, 0, s>>>(
+                  C.d, level_op(C), C.cc, C.x, C.w0, slot(res), res + 3);
+          });
           P27<double> P;
           for (int q = 0; q < 27; ++q)
             P.p[q] = C.P[q];
@@ -939,8 +1039,7 @@ int pmg_Vmgdriv_d(const int *iparm, const double *rparm, double *u,
                     (size_t)v.d.nx * v.d.ny);
   }
   const size_t nf = (size_t)D.lv[1].d.count();
-  D.rg0 = reduce_grid(D.lv[1].d);
-  const size_t nblk = (size_t)D.rg0.x * D.rg0.y * D.rg0.z;
+  const size_t nblk = reduce_blocks(D.lv, nlev);
   total += 3 * nf + 2 * nblk + 4;
   if (mgsolv == 1) {
     band_dims(D.lv[nlev].d, D.lv[nlev].kind, &D.bn, &D.bm, &D.blda);
@@ -1178,8 +1277,7 @@ int pmg_Vmvcs_d(int nx, int ny, int nz, double *x, const int *iz, double *w0,
   D.w3 = w3;
   // the reductions' partial sums, result slots and ticket
   cudaStream_t s = D.s;
-  D.rg0 = reduce_grid(D.lv[1].d);
-  const size_t nblk = (size_t)D.rg0.x * D.rg0.y * D.rg0.z;
+  const size_t nblk = reduce_blocks(D.lv, nlev);
   const size_t bytes = (2 * nblk + 4) * sizeof(double) + 64;
   PMG_CUDA_TRY(scratch_alloc(&D.block, bytes, s));
   PMG_CUDA_TRY(cudaMemsetAsync(D.block, 0, bytes, s));

@@ -316,14 +316,18 @@ int launch_cg_level(const Dims &d, const Op14<double> &A, const double *rhs,
                     double thresh, double rel_tol, int class_first_check,
                     int max_iters, int *status, cudaStream_t s) {
   if (cg_cluster_fits(d)) {
-    // levels up to 17^3: a cluster with the operator in shared memory
-    const size_t smem = cg_cluster_smem(d.nx, d.ny);
-    PMG_CUDA_TRY(set_smem_limit<cg_cluster_kernel>(
-        (int)cg_cluster_smem(kCgMaxN, kCgMaxN)));
-    cg_cluster_kernel<<<kCgCtas, kCgThreads, smem, s>>>(
-        d, A, rhs, x, thresh, rel_tol, class_first_check, max_iters, status);
-    PMG_LAUNCH_CHECK();
-    return PMG_OK;
+    // levels up to 17 points per axis: on chip for the whole solve
+    CgArgs a{};
+    a.d = d;
+    a.A = A;
+    a.rhs = rhs;
+    a.x = x;
+    a.thresh = thresh;
+    a.rel_tol = rel_tol;
+    a.class_first_check = class_first_check;
+    a.max_iters = max_iters;
+    a.status = status;
+    return launch_cg_on_chip<27, false>(a, s);
   }
   const long m = (long)(d.nx - 2) * (d.ny - 2) * (d.nz - 2);
   const int k = (int)((m + 1023) / 1024);
