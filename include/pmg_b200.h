@@ -679,12 +679,10 @@ int pmg_problem_coded_couplings(pmg_problem *p, int *coded);
 int pmg_problem_finest_streamed(pmg_problem *p, int *streamed);
 
 /* on != 0: choose kernels for many solves sharing the GPU rather than for
- * the latency of this one: the mixed path's lowest levels run in one CTA
- * instead of an 8-CTA cluster with its arrays in shared memory (a cluster
- * starts only when eight SMs of one GPC are idle at once). Same arithmetic
- * per point; the mixed results may differ in the last bits (sums in another
- * order). The serving runtime sets it on the problems it creates. Default
- * off. No reference counterpart. */
+ * the latency of this one. The kernels in use are the fastest for both, so
+ * the mode changes nothing today (results are the same bits); the serving
+ * runtime sets it on the problems it creates. Default off. No reference
+ * counterpart. */
 int pmg_problem_set_throughput_mode(pmg_problem *p, int on);
 
 /* Tile edge of the 27-point smoother, for the whole process. mode 1 (the

@@ -52,6 +52,12 @@ struct CgArgs {
   // sqrt(r0.r0)
   double thresh, rel_tol, errtol;
   int class_first_check;
+  // the class on level 1 of a V-cycle: a float right-hand side and result
+  // (mixed) and a start from zero; omega receives the damping of the result
+  const float *rhs32;
+  float *x32;
+  int zero_start;
+  double *omega;
   int max_iters;
   int *status; // [0] iterations, the class: [1] stopped by the cap
 };
@@ -112,23 +118,30 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
   const int lanes = cg_row_lanes(nx), mj = d.ny - 2;
   const int trow = tid / lanes, tplane = trow / mj;
   const bool own = tid - trow * lanes < mi && tplane < np;
-  const int i = own ? 2 + tid - trow * lanes : 2;
-  const int j = own ? 2 + trow - tplane * mj : 2;
-  const int k = own ? klo + tplane : klo;
-  const int gi = d.at(i, j, k);
-  const int sl = (k - klo + 1) * kCgPlane + (j - 1) * kCgRow + (i - 1);
+  const int i = 2 + tid - trow * lanes, j = 2 + trow - tplane * mj;
+  const int k = klo + tplane;
+  const int gi = own ? d.at(i, j, k) : 0;
+  // (idle lanes read their own columns of the padded rows, so that they meet
+  // no one else's bank, and discard them)
+  const int sl = (min(tplane, kPlanes - 1) + 1) * kCgPlane +
+                 (j - 1) * kCgRow + (i - 1);
   StencilRow<double, KIND> row;
   row.clear();
-  double xv = 0.0, rv = 0.0, pv = 0.0, apv = 0.0;
+  double fv = 0.0, xv = 0.0, rv = 0.0, pv = 0.0, apv = 0.0;
   if (own) {
     row.load(a.A, a.cc, gi, nx, nx * d.ny);
-    xv = a.x[gi];
     const double *x = a.x;
     const int sy = nx, sz = nx * d.ny;
     auto xval = [&](int dx, int dy, int dz) {
       return x[gi + dx + dy * sy + dz * sz];
     };
-    rv = APBS ? row.resid(a.rhs[gi], xval) : a.rhs[gi] - row.apply(xval);
+    fv = !APBS && a.rhs32 ? (double)a.rhs32[gi] : a.rhs[gi];
+    if (!APBS && a.zero_start) {
+      rv = fv;
+    } else {
+      xv = x[gi];
+      rv = APBS ? row.resid(fv, xval) : fv - row.apply(xval);
+    }
   }
   auto pval = [&](int dx, int dy, int dz) {
     return sP[sl + dx + dy * kCgRow + dz * kCgPlane];
@@ -166,10 +179,8 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     __syncthreads();
   }
   auto push = [&]() {
-    if (dn_bar)
-      send(dn, rv, dn_bar);
-    if (up_bar)
-      send(up, rv, up_bar);
+    send(dn, rv, dn_bar);
+    send(up, rv, up_bar);
   };
   // the points of the two copied planes this thread keeps (at most two)
   int h0 = -1, h1 = -1; // entry in sR, or -1
@@ -208,13 +219,11 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     }
     v = (s[0] + s[1]) + (s[2] + s[3]);
     if constexpr (C > 1) {
-      if (warp == 0 && lane < C)
-        send(cluster_addr(&sCta[set][rank], lane), v,
-             cluster_addr(&bar[set], lane));
+      send(cluster_addr(&sCta[set][rank], lane & (C - 1)), v,
+           tid < C ? cluster_addr(&bar[set], lane & (C - 1)) : 0u);
       lost |= !mbar_wait_cluster(&bar[set], parity[set]);
       parity[set] ^= 1u;
-      if (tid == 0)
-        mbar_expect_tx(&bar[set], msg_bytes[set]);
+      mbar_expect_tx_if(tid == 0, &bar[set], msg_bytes[set]);
       const double *t = sCta[set];
       v = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
       static_assert(C == 8, "the tree of the CTAs' sums");
@@ -268,8 +277,8 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
       }
     }
     pv = pnew;
-    if (own)
-      apv = row.apply(pval);
+    // (every lane: threads without a point hold a row of zeros)
+    apv = row.apply(pval);
     const double pap = allsum(apv * pv, 1);
     if (!APBS && it == 0) {
       if (C > 1 && __syncthreads_or(lost))
@@ -290,8 +299,32 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     rs_old = rs;
     rs = allsum(rv * rv, 0);
   }
+  if constexpr (!APBS)
+    if (a.omega) {
+      // the damping (f . x) / (x . A x), x exchanged like r. (The sums'
+      // sets alternate: the last one was r.r unless no iteration ran.)
+      if (it > 0)
+        allsum(0.0, 1);
+      rv = xv;
+      push();
+      const double up_sum = allsum(fv * xv, 0);
+      if (own)
+        sP[sl] = xv;
+      if constexpr (C > 1) {
+        if (h0 >= 0)
+          sP[copy_at(h0)] = sR[h0];
+        if (h1 >= 0)
+          sP[copy_at(h1)] = sR[h1];
+      }
+      __syncthreads();
+      const double lo_sum = allsum(own ? xv * row.apply(pval) : 0.0, 1);
+      if (rank == 0 && tid == 0)
+        *a.omega = up_sum / lo_sum;
+    }
   if (own) {
-    if (!APBS || it > 0)
+    if (!APBS && a.x32)
+      a.x32[gi] = (float)xv;
+    else if (!APBS || it > 0)
       a.x[gi] = xv;
     if constexpr (APBS) {
       a.r[gi] = rv;
@@ -307,8 +340,10 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     if constexpr (!APBS)
       a.status[1] = capped || lost ? 1 : 0;
   }
-  if constexpr (C > 1)
-    cgs::this_cluster().sync(); // no CTA leaves while another stores to it
+  if constexpr (C > 1) {
+    settle_if(lost);
+    cgs::this_cluster().sync(); // no CTA leaves while another sends to it
+  }
 }
 
 template <int KIND, bool APBS>

@@ -134,9 +134,6 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src,
                : "memory");
 }
 
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-}
 
 // Sub-colour step S (points (i, j) with i % 2 = S & 1, j % 2 = S >> 1) with
 // halo H of a TI x TJ tile: a fixed NUX x NUY grid of the points within H of

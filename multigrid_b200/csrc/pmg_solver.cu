@@ -12,7 +12,6 @@
 
 #include "build_kernels.cuh"
 #include "bottom_cluster.cuh"
-#include "bottom_cycle.cuh"
 #include "gs27_tiled.cuh"
 #include "gs27_tma.cuh"
 #include "gs7_stream.cuh"
@@ -191,6 +190,10 @@ struct pmg_problem {
   LevelBuf lv[kMaxLevels + 1];
   double *cg_r = nullptr, *cg_p = nullptr, *cg_ap = nullptr;
   int *cg_status = nullptr;
+  // refinement paths with a small level 1 below the one-launch levels: the
+  // inverse of its operator (bottom_cluster.cuh) and whether it is good
+  double *inv1 = nullptr;
+  int *inv1_ok = nullptr;
   // device: set by the staged kernels (gs27_tma_kernel, gs7_stream_kernel,
   // defect_norm_stream_kernel) on a lost stage
   int *kernel_err = nullptr;
@@ -198,8 +201,8 @@ struct pmg_problem {
   // Relative stopping threshold of the coarsest CG on the mixed path's
   // correction equation (the FP64 path keeps the class's absolute 1e-8).
   double coarse_rtol = 1e-4;
-  // Mixed path: levels 1 .. bottom_top (n <= 17) run in one CTA
-  // (bottom_cycle_kernel); 0 when level 1 is too large.
+  // Levels 1 .. bottom_top (n <= 17) run in one launch
+  // (bottom_cluster.cuh); 0: each level by itself.
   int bottom_top = 0;
   // pmg_set_tma_staging when the problem was created (read once, so that
   // both passes of plan() lay out the same arrays)
@@ -219,7 +222,6 @@ struct pmg_problem {
   cudaEvent_t done_ev = nullptr;
   bool solve_pending = false;
   bool host_loop = false; // pmg_problem_set_host_loop
-  bool throughput = false; // pmg_problem_set_throughput_mode
   bool use_codes = true;   // pmg_problem_set_coded_couplings
   // the finest colour passes stream their rows through shared memory
   // (gs7_stream.cuh); fixed at creation by pmg_set_finest_streaming
@@ -282,15 +284,18 @@ void launch_ideal_lambda(const Dims &d, const Op14<T> &A, const T *x,
   }
 }
 
-// Mixed path: the top level of the one-launch bottom cycle (the levels up
-// to 17 points per axis); 0 on the other paths.
-int bottom_top_of(int base, int nlev, int precision) {
+// The top level of the one-launch bottom cycle: the finest coarse level of
+// up to 17 points per axis over levels of up to 9; 0 when that is level 1 (a
+// launch of its own, cg_cluster.cuh) or the levels do not fit.
+int bottom_top_of(int base, int nlev) {
   int top = 0;
-  if (precision == PMG_PREC_MIXED)
-    for (int L = 1; L < nlev && L <= kBottomMaxLevels; ++L)
-      if (level_n(base, L) <= kBottomMaxN)
-        top = L;
-  return top;
+  for (int L = 1; L < nlev && L <= kBottomMaxLevels; ++L)
+    if (level_n(base, L) <= kBottomMaxN)
+      top = L;
+  return top >= 2 && top - 2 <= kBlMaxLevels &&
+                 level_n(base, top - 1) <= kBlMaxN
+             ? top
+             : 0;
 }
 
 // Lays out every device array of a problem; with a.base == nullptr only
@@ -302,14 +307,14 @@ void plan(pmg_problem *p, Arena &a) {
   // of x and f, converted at the level's V-cycle)
   const bool fast = p->precision == PMG_PREC_FP64_FAST ||
                     p->precision == PMG_PREC_FP64;
-  const int bottom_top = bottom_top_of(p->base, p->nlev, p->precision);
+  const int bottom_top = bottom_top_of(p->base, p->nlev);
   for (int L = 1; L <= p->nlev; ++L) {
     LevelBuf &v = p->lv[L];
     v.n = level_n(p->base, L);
     v.d = Dims{v.n, v.n, v.n};
     v.n3 = v.d.count();
     const bool fine = L == p->nlev;
-    const bool pitched = mixed && !fine && L > bottom_top;
+    const bool pitched = mixed && !fine && L > std::max(bottom_top, 1);
     v.d32 = pitched ? Dims{v.n, v.n, v.n, (v.n + 3) & ~3} : v.d;
     v.n3_32 = v.d32.count();
     const int nops = fine ? 4 : 14;
@@ -374,6 +379,12 @@ void plan(pmg_problem *p, Arena &a) {
   p->cg_ap = a.take<double>(n1);
   p->cg_status = a.take<int>(2);
   p->kernel_err = a.take<int>(1);
+  const long m1 = (long)(p->lv[1].n - 2) * (p->lv[1].n - 2) *
+                  (p->lv[1].n - 2);
+  if (bottom_top > 0 && p->precision != PMG_PREC_FP64 && m1 <= kInvMax) {
+    p->inv1 = a.take<double>(kInvMax * kInvMax);
+    p->inv1_ok = a.take<int>(1);
+  }
   p->d_state = a.take<SolveState>(1);
   // partials of the largest launch using each slot: the finest level's
   // reductions, and the damping on any coarse level
@@ -477,17 +488,106 @@ int smooth64(pmg_problem *p, int L, int nsweeps, int zero_init,
 }
 
 // Coarsest level: the class's CG (absolute 1e-8, first test on
-// sqrt(sqrt(r.r))) on the FP64 path; on the refinement paths (mixed,
-// fp64-fast) a zero-started CG to coarse_rtol relative to its initial
-// residual.
-int cg_level1(pmg_problem *p, const double *rhs, double *x) {
+// sqrt(sqrt(r.r)), from the last cycle's x) on the FP64 path; on the
+// refinement paths (mixed, fp64-fast) a zero-started CG to coarse_rtol
+// relative to its initial residual. One launch leaves x and the level's
+// damping where the level fits on chip (cg_cluster.cuh); else the mixed path
+// converts its float right-hand side and result, and the damping is a launch
+// of its own.
+int cg_level1(pmg_problem *p) {
   LevelBuf &v = p->lv[1];
-  if (p->precision != PMG_PREC_FP64)
-    return launch_cg_level(v.d, v.A64(14), rhs, x, p->cg_r, p->cg_p,
-                           p->cg_ap, 0.0, p->coarse_rtol, 0, kCgMaxIters,
-                           p->cg_status, p->stream);
-  return launch_cg_level(v.d, v.A64(14), rhs, x, p->cg_r, p->cg_p, p->cg_ap,
-                         1e-8, 0.0, 1, kCgMaxIters, p->cg_status, p->stream);
+  const bool fp64 = p->precision == PMG_PREC_FP64;
+  const bool mixed = p->precision == PMG_PREC_MIXED;
+  const double thresh = fp64 ? 1e-8 : 0.0, rtol = fp64 ? 0.0 : p->coarse_rtol;
+  cudaStream_t s = p->stream;
+  if (cg_cluster_fits(v.d)) {
+    CgArgs a{};
+    a.d = v.d;
+    a.A = v.A64(14);
+    a.rhs = v.f;
+    a.x = v.x;
+    a.rhs32 = mixed ? v.f32 : nullptr;
+    a.x32 = mixed ? v.x32 : nullptr;
+    a.zero_start = !fp64;
+    a.omega = v.omega;
+    a.thresh = thresh;
+    a.rel_tol = rtol;
+    a.class_first_check = fp64;
+    a.max_iters = kCgMaxIters;
+    a.status = p->cg_status;
+    return launch_cg_on_chip<27, false>(a, s);
+  }
+  if (mixed)
+    convert_kernel<float, double><<<flat_grid(v.n3), 256, 0, s>>>(v.n3, v.f32,
+                                                                  v.f);
+  if (!fp64)
+    PMG_CUDA_TRY(cudaMemsetAsync(v.x, 0, sizeof(double) * v.n3, s));
+  const int rc = launch_cg_level(v.d, v.A64(14), v.f, v.x, p->cg_r, p->cg_p,
+                                 p->cg_ap, thresh, rtol, fp64, kCgMaxIters,
+                                 p->cg_status, s);
+  if (rc)
+    return rc;
+  launch_ideal_lambda<double>(v.d, v.A64(14), v.x, v.f, p->red_lambda,
+                              v.omega, s);
+  if (mixed)
+    convert_kernel<double, float><<<flat_grid(v.n3), 256, 0, s>>>(v.n3, v.x,
+                                                                  v.x32);
+  PMG_LAUNCH_CHECK();
+  return PMG_OK;
+}
+
+// Arguments of the one-launch cycle over levels 1 .. top.
+template <typename T> BottomArgs<T> bottom_args(pmg_problem *p, int top) {
+  using Arr = LevelArrays<T>;
+  const bool fp64 = p->precision == PMG_PREC_FP64;
+  BottomArgs<T> a{};
+  a.top = top;
+  for (int L = 1; L <= top; ++L) {
+    LevelBuf &v = p->lv[L];
+    BottomLevel<T> &b = a.lv[L];
+    b.d = v.d;
+    if (L > 1)
+      b.A = Arr::A(v);
+    b.P = Arr::P(v);
+    b.x = Arr::x(v);
+    b.f = Arr::f(v);
+    b.omega = v.omega;
+  }
+  a.A1 = p->lv[1].A64(14);
+  a.x1 = p->lv[1].x;
+  a.thresh = fp64 ? 1e-8 : 0.0;
+  a.rtol = fp64 ? 0.0 : p->coarse_rtol;
+  a.class_first_check = fp64;
+  a.warm_start = fp64;
+  a.max_iters = kCgMaxIters;
+  a.status = p->cg_status;
+  a.kernel_err = p->kernel_err;
+  a.inv = p->inv1;
+  a.inv_ok = p->inv1_ok;
+  return a;
+}
+
+// Levels 1 .. top of the V-cycle in one launch (bottom_cluster.cuh).
+template <typename T> int launch_bottom(pmg_problem *p, int top) {
+  const BottomArgs<T> a = bottom_args<T>(p, top);
+  cudaStream_t s = p->stream;
+  if (!bc_fits(a)) {
+    set_last_message("launch_bottom: levels do not fit");
+    return PMG_ERR_STATE;
+  }
+  if constexpr (sizeof(T) == sizeof(float)) {
+    PMG_CUDA_TRY(set_smem_limit<bottom_cluster_f_kernel>(
+        (int)sizeof(BcSmem<float>)));
+    bottom_cluster_f_kernel<<<kCgCtas, kBcThreads, sizeof(BcSmem<float>),
+                              s>>>(a);
+  } else {
+    PMG_CUDA_TRY(set_smem_limit<bottom_cluster_d_kernel>(
+        (int)sizeof(BcSmem<double>)));
+    bottom_cluster_d_kernel<<<kCgCtas, kBcThreads, sizeof(BcSmem<double>),
+                              s>>>(a);
+  }
+  PMG_LAUNCH_CHECK();
+  return PMG_OK;
 }
 
 // v_cycle of the class (PBE_pmgc_class.h:1070-1114) on level L.
@@ -497,7 +597,7 @@ int vcycle64(pmg_problem *p, int L, int as_preconditioner) {
   const int sl = L * 8;
   if (L == 1) {
     prof_begin(p, sl + kPhCoarse);
-    int rc = cg_level1(p, v.f, v.x);
+    int rc = cg_level1(p);
     prof_end(p, sl + kPhCoarse);
     return rc;
   }
@@ -541,11 +641,21 @@ int vcycle64(pmg_problem *p, int L, int as_preconditioner) {
                                                        c.Pc());
   prof_end(p, sl + kPhRestrict);
   PMG_LAUNCH_CHECK();
-  if ((rc = vcycle64(p, L - 1, 0)))
+  // levels 1 .. bottom_top in one launch; it, and level 1 by itself, also
+  // leave the level's damping
+  const bool bottom_below = L - 1 <= p->bottom_top;
+  if (bottom_below) {
+    prof_begin(p, sl + kPhCoarse);
+    if ((rc = launch_bottom<double>(p, L - 1)))
+      return rc;
+    prof_end(p, sl + kPhCoarse);
+  } else if ((rc = vcycle64(p, L - 1, 0))) {
     return rc;
+  }
   prof_begin(p, sl + kPhLambda);
-  launch_ideal_lambda<double>(c.d, c.A64(14), c.x, c.f, p->red_lambda,
-                              c.omega, s);
+  if (!bottom_below && L - 1 > 1)
+    launch_ideal_lambda<double>(c.d, c.A64(14), c.x, c.f, p->red_lambda,
+                                c.omega, s);
   prof_end(p, sl + kPhLambda);
   // x += w * (interpolated correction), one pass
   prof_begin(p, sl + kPhInterp);
@@ -802,52 +912,6 @@ int smooth_ref(pmg_problem *p, int L, int nsweeps, int zero_init, T **cur) {
                            nsweeps, 0, zero_init, p->stream, cur);
 }
 
-// Arguments of the one-CTA cycle over levels 1 .. top.
-BottomArgs bottom_args(pmg_problem *p, int top) {
-  BottomArgs a{};
-  a.top = top;
-  for (int L = 1; L <= top; ++L) {
-    LevelBuf &v = p->lv[L];
-    BottomLevel &b = a.lv[L];
-    b.d = v.d;
-    b.A = v.A32(L > 1 ? 14 : 0);
-    b.P = v.Pc32();
-    b.x = v.x32;
-    b.f = v.f32;
-    b.r = v.r32;
-    b.omega = v.omega;
-  }
-  a.A1 = p->lv[1].A64(14);
-  a.x1 = p->lv[1].x;
-  a.f1 = p->lv[1].f;
-  a.cg_r = p->cg_r;
-  a.cg_p = p->cg_p;
-  a.cg_ap = p->cg_ap;
-  a.rtol = p->coarse_rtol;
-  a.max_iters = kCgMaxIters;
-  a.status = p->cg_status;
-  return a;
-}
-
-// Levels 1 .. top of the mixed V-cycle in one launch: on a cluster with
-// every array in shared memory when they fit (bottom_cluster.cuh), else, or
-// in throughput mode, in one CTA out of global memory (bottom_cycle.cuh).
-// The cluster is faster for a solve alone, but it can start only when eight
-// SMs of one GPC are idle at once, which many concurrent solves rarely
-// leave (measured: serving saturation 111 against 133 solves/s).
-int launch_bottom(pmg_problem *p, int top) {
-  const BottomArgs a = bottom_args(p, top);
-  cudaStream_t s = p->stream;
-  if (!p->throughput && bc_fits(a)) {
-    PMG_CUDA_TRY(set_smem_limit<bottom_cluster_kernel>((int)kBcMaxSmem));
-    bottom_cluster_kernel<<<kCgCtas, kBcThreads, bc_layout(a).total, s>>>(a);
-  } else {
-    bottom_cycle_kernel<<<1, 1024, 0, s>>>(a);
-  }
-  PMG_LAUNCH_CHECK();
-  return PMG_OK;
-}
-
 // V-cycle in type T on the correction equation, every level zero-started
 // (v_cycle with as_preconditioner, PBE_pmgc_class.h:1070-1114); level 1 in
 // double. T = float is the mixed path, T = double fp64-fast.
@@ -859,11 +923,7 @@ template <typename T> int vcycle_ref(pmg_problem *p, int L) {
   const int sl = L * 8;
   if (L == 1) {
     prof_begin(p, sl + kPhCoarse);
-    if (kFloat)
-      convert_kernel<float, double><<<flat_grid(v.n3), 256, 0, s>>>(
-          v.n3, v.f32, v.f);
-    PMG_CUDA_TRY(cudaMemsetAsync(v.x, 0, sizeof(double) * v.n3, s));
-    int rc = cg_level1(p, v.f, v.x);
+    int rc = cg_level1(p);
     prof_end(p, sl + kPhCoarse);
     return rc;
   }
@@ -871,7 +931,7 @@ template <typename T> int vcycle_ref(pmg_problem *p, int L) {
   const int kind = L == p->nlev ? 7 : 27;
   int rc;
   T *x = A::x(v);
-  const bool bottom_below = kFloat && L - 1 <= p->bottom_top;
+  const bool bottom_below = L - 1 <= p->bottom_top;
   prof_begin(p, sl + kPhPre);
   if ((rc = smooth_ref<T>(p, L, 2, 1, &x)))
     return rc;
@@ -907,9 +967,9 @@ template <typename T> int vcycle_ref(pmg_problem *p, int L) {
   prof_end(p, sl + kPhRestrict);
   PMG_LAUNCH_CHECK();
   if (bottom_below) {
-    // levels 1 .. L-1 in one CTA; it also leaves the damping of level L-1
+    // levels 1 .. L-1 in one launch; it also leaves the damping of level L-1
     prof_begin(p, sl + kPhCoarse);
-    if ((rc = launch_bottom(p, L - 1)))
+    if ((rc = launch_bottom<T>(p, L - 1)))
       return rc;
     prof_end(p, sl + kPhCoarse);
     PMG_LAUNCH_CHECK();
@@ -917,18 +977,10 @@ template <typename T> int vcycle_ref(pmg_problem *p, int L) {
     return rc;
   }
   prof_begin(p, sl + kPhLambda);
-  if (bottom_below) {
-    // damping computed by the bottom kernel
-  } else if (L - 1 == 1) {
-    launch_ideal_lambda<double>(c.d, c.A64(14), c.x, c.f, p->red_lambda,
-                                c.omega, s);
-    if (kFloat)
-      convert_kernel<double, float><<<flat_grid(c.n3), 256, 0, s>>>(
-          c.n3, c.x, c.x32);
-  } else {
+  // (the bottom launch and level 1 by itself leave theirs)
+  if (!bottom_below && L - 1 > 1)
     launch_ideal_lambda<T>(A::dims(c), A::A(c), A::x(c), A::f(c),
                            p->red_lambda, c.omega, s);
-  }
   prof_end(p, sl + kPhLambda);
   // x += w * (interpolated correction), one pass
   prof_begin(p, sl + kPhInterp);
@@ -1530,7 +1582,7 @@ int pmg_problem_create(int base, int nlev, double box, int precision,
   p->nlev = nlev;
   p->box = box;
   p->precision = precision;
-  p->bottom_top = bottom_top_of(base, nlev, precision);
+  p->bottom_top = bottom_top_of(base, nlev);
   p->tma_on = !tma_disabled();
   Arena a;
   plan(p, a);
@@ -1685,9 +1737,7 @@ int pmg_problem_finest_streamed(pmg_problem *p, int *streamed) {
 int pmg_problem_set_throughput_mode(pmg_problem *p, int on) {
   if (!p)
     return PMG_ERR_ARG;
-  if ((bool)on != p->throughput)
-    drop_graphs(p); // the captured cycles bake the kernel choice in
-  p->throughput = on != 0;
+  (void)on; // one set of kernels serves both (bottom_cluster.cuh)
   return PMG_OK;
 }
 
@@ -1805,6 +1855,12 @@ int pmg_build_hierarchy(pmg_problem *p, int trilinear) {
                             f.A64(kind == 7 ? 4 : 14), out, s, out32,
                             &c.d32)))
       return rc;
+  }
+  if (p->inv1) {
+    level1_inverse_kernel<<<1, 1024, 0, s>>>(p->lv[1].d, p->lv[1].A64(14),
+                                            p->inv1, p->inv1_ok);
+    PMG_LAUNCH_CHECK();
+    ++p->launches;
   }
   if (mixed) {
     LevelBuf &v = p->lv[p->nlev];

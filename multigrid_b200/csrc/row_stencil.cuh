@@ -79,6 +79,27 @@ template <typename T, int KIND> struct StencilRow {
       return s + centre * v(0, 0, 0);
     }
   }
+  // A v with fused products and four shorter chains, for the solves that are
+  // held to rounding and not to bits
+  template <class V> __device__ __forceinline__ T apply_fused(V v) const {
+    T s[4] = {centre * v(0, 0, 0), T(0), T(0), T(0)};
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      const Offset3 e = neighbour<KIND>(t);
+      s[t & 3] = fma(-c[t], v(e.x, e.y, e.z), s[t & 3]);
+    }
+    return (s[0] + s[1]) + (s[2] + s[3]);
+  }
+  // f + neighbour sums, fused in four chains
+  template <class V> __device__ __forceinline__ T fused_sum(T f, V v) const {
+    T s[4] = {f, T(0), T(0), T(0)};
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      const Offset3 e = neighbour<KIND>(t);
+      s[t & 3] = fma(c[t], v(e.x, e.y, e.z), s[t & 3]);
+    }
+    return (s[0] + s[1]) + (s[2] + s[3]);
+  }
   // f - A v in the order of resid_at (Vmresid7_1s, Vmresid27_1s)
   template <class V> __device__ __forceinline__ T resid(T f, V v) const {
     if constexpr (KIND == 27) {

@@ -229,8 +229,8 @@ class PBELinearProblem:
 
     def set_throughput_mode(self, on: bool = True) -> None:
         """Choose kernels for many solves sharing the GPU (the serving
-        runtime's setting) rather than for this solve's latency; mixed
-        results may differ from the default mode in the last bits."""
+        runtime's setting) rather than for this solve's latency; today one
+        set of kernels serves both (the same bits)."""
         _lib.check("pmg_problem_set_throughput_mode",
                    _lib.lib.pmg_problem_set_throughput_mode(self._h, int(on)))
 

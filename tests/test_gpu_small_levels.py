@@ -85,3 +85,32 @@ def test_class_cg_sizes(restatement, n):
     it = pmgc.cg_level(n, n, n, [T(a) for a in ops], T(f), x)
     assert it == it_o > 0
     assert rel(x.cpu().numpy(), xo) <= 1e-12
+
+
+# hierarchies whose levels of up to 17^3 run in one launch: 9^3 over 5^3, two
+# and three levels below the top, a 3^3 coarsest level, 13^3 over 7^3 (125
+# unknowns), 17^3 over 9^3 (343 unknowns); and whose level 1 (13^3, 19^3) runs
+# by itself, on chip and not
+@pytest.mark.parametrize("base,nlev", [(2, 3), (2, 4), (1, 5), (3, 3), (4, 3),
+                                       (6, 2), (9, 2)])
+def test_low_levels_of_the_cycle(restatement, base, nlev):
+    """FP64 against the restated class: the same cycles, the potential to
+    1e-12 (sums in another order); the refinement paths to 1e-8 of it."""
+    from multigrid_b200 import PBELinearProblem
+    from multigrid_b200.molecule import Workload, level_n
+    from multigrid_b200.problem import setup_fine
+    n = level_n(base, nlev)
+    w = Workload("shape", base, nlev, 0.8, 12, 0.25 * 0.8 * (n - 1), 11)
+    fine = setup_fine(w.n, w.h, w.atoms(), w.physics)
+    xo, co, _ = restatement.solve(base, nlev, fine, tol=1e-10, max_cycles=100)
+    for prec, tol in (("fp64", 1e-12), ("fp64-fast", 1e-8), ("mixed", 1e-8)):
+        with PBELinearProblem(base, nlev, w.box, prec, w.physics,
+                              hierarchy="reference") as p:
+            p.set_fine(**fine)
+            p.buildmultilevelops()
+            r = p.solve(tol=1e-10, max_cycles=100)
+            x = p.potential().ravel()
+        assert r.relres < 1e-10, (prec, r.cycles, r.relres)
+        assert np.linalg.norm(x - xo) <= tol * np.linalg.norm(xo), prec
+        if prec == "fp64":
+            assert r.cycles == co
