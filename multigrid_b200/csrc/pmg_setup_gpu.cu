@@ -16,9 +16,9 @@
 //             stable sort over records generated in atom order, and each
 //             point sums its run in that order: the host's serial sum, bit
 //             for bit.
-//   boundary  the multiple Debye-Hueckel sum over atoms in order on the six
-//             faces; exp() is CUDA's, so values agree with the host's to a
-//             few ulp.
+//   boundary  the multiple Debye-Hueckel sum over atoms on the six faces, in
+//             another order than the host's and with its own exp and square
+//             root: equal to a few ulp of the sum's largest terms.
 // All work is stream-ordered on the caller's stream; scratch comes from the
 // library's stream-ordered pool.
 #include <cub/device/device_radix_sort.cuh>
@@ -39,27 +39,27 @@ constexpr int kSetupThreads = 256;
 struct SphereSet {
   const double *centers; // rows of `stride` doubles, x y z first
   int stride;
-  int count;
+  int count;            // (an upper bound where count_dev is given)
   const double *radius; // radius of row q at radius[q * stride] or null
   double radius_add;    // added to the row radius (or the radius if null)
-  const unsigned char *use; // row q used only when use[q] != 0 (or null)
-  int axis;                 // centre shifted by -h/2 along this axis (-1: no)
+  const int *count_dev; // the count, on the device (or null)
+  unsigned char *mask;  // set to 1 at the marked points
+};
+// Up to three sets marked by one launch.
+struct SphereSets {
+  SphereSet set[3];
+  int axis; // centres shifted by -h/2 along this axis (-1: no)
 };
 
-// Marks the grid points of every sphere of a set (for_dots_in_sphere of the
-// host set-up): axis-0 range ceil((c0 - r)/h) .. trunc((c0 + r)/h), chord
-// half-widths from sqrt of the clamped squared remainders on axes 1 and 2.
-// One block per sphere; threads over the (i0, i1) bounding rectangle.
-template <typename M>
-__global__ void __launch_bounds__(kSetupThreads)
-    mark_spheres_kernel(int n, double h, SphereSet set, M *mask, M value) {
-  const int q = blockIdx.x;
-  if (q >= set.count || (set.use && !set.use[q]))
-    return;
+// The points of sphere q of a set, by one warp.
+__device__ __forceinline__ void mark_sphere(int n, double h,
+                                            const SphereSet &set, int axis,
+                                            int q, int lane) {
   const double *row = set.centers + (size_t)q * set.stride;
-  double c[3] = {row[0], row[1], row[2]};
-  if (set.axis >= 0)
-    c[set.axis] -= 0.5 * h;
+  const double hx = 0.5 * h;
+  const double c[3] = {axis == 0 ? row[0] - hx : row[0],
+                       axis == 1 ? row[1] - hx : row[1],
+                       axis == 2 ? row[2] - hx : row[2]};
   const double r = set.radius ? set.radius[(size_t)q * set.stride] +
                                     set.radius_add
                               : set.radius_add;
@@ -70,8 +70,10 @@ __global__ void __launch_bounds__(kSetupThreads)
   const int w0 = hi0 - lo0 + 1, w1 = bhi1 - blo1 + 1;
   if (w0 <= 0 || w1 <= 0)
     return;
-  for (int t = threadIdx.x; t < w0 * w1; t += blockDim.x) {
+  for (int t = lane; t < w0 * w1; t += 32) {
     const int i0 = lo0 + t / w1, i1 = blo1 + t % w1;
+    if (i0 < 0 || i1 < 0 || i0 >= n || i1 >= n)
+      continue;
     double s1 = r * r - ((c[0] - h * i0) * (c[0] - h * i0));
     if (s1 < 0)
       s1 = 0;
@@ -87,11 +89,45 @@ __global__ void __launch_bounds__(kSetupThreads)
     const double ww2 = sqrt(s2);
     const int lo2 = (int)ceil((c[2] - ww2) / h);
     const int hi2 = (int)((c[2] + ww2) / h);
-    if (i0 < 0 || i1 < 0 || i0 >= n || i1 >= n)
-      continue;
+    unsigned char *m = set.mask + ((size_t)i0 * n + i1) * n;
     for (int i2 = lo2 < 0 ? 0 : lo2; i2 <= hi2 && i2 < n; ++i2)
-      mask[((size_t)i0 * n + i1) * n + i2] = value;
+      m[i2] = 1;
   }
+}
+
+// Marks the grid points of every sphere of the sets (for_dots_in_sphere of
+// the host set-up): axis-0 range ceil((c0 - r)/h) .. trunc((c0 + r)/h), chord
+// half-widths from sqrt of the clamped squared remainders on axes 1 and 2.
+// One warp per sphere, lanes over the (i0, i1) bounding rectangle (~60 points
+// of a probe sphere); the warps of a grid that fills the GPU once stride over
+// the spheres. A block per sphere, with the probe positions that are not free
+// among them, spent its time starting blocks (3000 atoms, 129^3: 850 -> 216 us
+// for all marks, with the three sets of an axis in one launch; a warp per
+// sphere with the unfree ones skipped, 272 us).
+__global__ void __launch_bounds__(kSetupThreads)
+    mark_spheres_kernel(int n, double h, SphereSets sets) {
+  const int lane = threadIdx.x & 31;
+  const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+  int count[3];
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+    count[t] =
+        sets.set[t].count_dev ? *sets.set[t].count_dev : sets.set[t].count;
+  for (int g = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+       g < count[0] + count[1] + count[2]; g += warps) {
+    if (g < count[0])
+      mark_sphere(n, h, sets.set[0], sets.axis, g, lane);
+    else if (g < count[0] + count[1])
+      mark_sphere(n, h, sets.set[1], sets.axis, g - count[0], lane);
+    else
+      mark_sphere(n, h, sets.set[2], sets.axis, g - count[0] - count[1],
+                  lane);
+  }
+}
+unsigned mark_blocks(const SphereSets &s) {
+  const long q = (long)s.set[0].count + s.set[1].count + s.set[2].count;
+  const long b = (q * 32 + kSetupThreads - 1) / kSetupThreads;
+  return (unsigned)std::min(b, 148L * 8);
 }
 
 __global__ void face_from_masks_kernel(long count, const unsigned char *inside,
@@ -176,7 +212,8 @@ __global__ void charge_sum_kernel(const double *atoms, int nrec, double h,
 
 // Probe centres on the sphere of radius r_a + probe around every atom; a
 // centre is kept when no other inflated sphere contains it
-// (d^2 < R_b^2 (1 - 1e-12), the host's test). Output rows (x, y, z). The
+// (d^2 < R_b^2 (1 - 1e-12), the host's test). Output: the kept centres as rows
+// (x, y, z), in any order (their marks do not depend on it), *kept of them. The
 // atoms are found through a cell list: a centre lies within the largest
 // inflated radius (<= the cell edge) of any sphere containing it, so only
 // the 27 cells around it are searched; "kept" is an AND over atoms, so the
@@ -185,7 +222,7 @@ __global__ void __launch_bounds__(kSetupThreads)
     probe_centres_cells_kernel(const double *atoms, int natoms, double probe,
                                const ProbeDir *dirs, double cell, int dim,
                                const int *cell_start, const int *cell_atoms,
-                               double *centres, unsigned char *free_flag) {
+                               double *centres, int *kept) {
   const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (g >= (long)natoms * kProbePoints)
     return;
@@ -224,10 +261,12 @@ __global__ void __launch_bounds__(kSetupThreads)
           }
         }
       }
-  centres[3 * g + 0] = pc[0];
-  centres[3 * g + 1] = pc[1];
-  centres[3 * g + 2] = pc[2];
-  free_flag[g] = free ? 1 : 0;
+  if (!free)
+    return;
+  const int slot = atomicAdd(kept, 1);
+  centres[3 * slot + 0] = pc[0];
+  centres[3 * slot + 1] = pc[1];
+  centres[3 * slot + 2] = pc[2];
 }
 
 // Cell list of the atoms: cell of each atom and per-cell counts
@@ -251,55 +290,158 @@ __global__ void atom_scatter_kernel(int natoms, const int *cid, int *fill,
     cell_atoms[atomicAdd(&fill[cid[a]], 1)] = a;
 }
 
-// Multiple Debye-Hueckel values on the six faces (atoms in order); faces
-// share their edges, which get the same value from each.
-__global__ void __launch_bounds__(kSetupThreads)
-    boundary_kernel(const double *atoms, int natoms, int n, double h,
-                    double pref, double kappa, double *x0) {
-  __shared__ double sa[kSetupThreads * 5];
-  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long face_pts = (long)n * n;
-  const bool active = g < 6 * face_pts;
-  long i0 = 0, i1 = 0, i2 = 0;
-  if (active) {
-    const int face = (int)(g / face_pts);
-    const long q = g % face_pts;
-    const long a = q / n, b = q % n;
-    switch (face) {
-    case 0: i0 = a; i1 = b; i2 = 0; break;
-    case 1: i0 = a; i1 = b; i2 = n - 1; break;
-    case 2: i0 = 0; i1 = a; i2 = b; break;
-    case 3: i0 = n - 1; i1 = a; i2 = b; break;
-    case 4: i0 = a; i1 = 0; i2 = b; break;
-    default: i0 = a; i1 = n - 1; i2 = b; break;
-    }
+// ---- multiple Debye-Hueckel boundary ----------------------------------------
+// x0(p) = sum over atoms of f_a exp(-kappa (d - r_a)) / d on the six faces,
+// f_a = q / (pref (1 + kappa r_a)). 10^8 to 10^9 terms in double, bound by the
+// FP64 units: with CUDA's sqrt, exp and divide a term is ~88 of their
+// operations. Here it is ~27:
+//   * a thread takes kDhPoints points of one face row, which share two of the
+//     three squared distances;
+//   * 1 / d from the hardware's reciprocal square root estimate and one
+//     third-order correction (relative error e -> O(e^3), e <= 2^-20), d as
+//     d^2 / d;
+//   * exp by a table of 2^(j/64) and a degree-5 polynomial (Tang, ACM TOMS
+//     15, 1989): y = d' (-kappa 64 / ln 2) = m + f, the product in two parts
+//     so that f keeps its last bits, exp = 2^(m/64) e^(f ln 2 / 64).
+// The block's eight warps take the same points and every eighth atom each;
+// their sums are added in warp order (deterministic; without that split a
+// 65^3 grid has too few points to fill the GPU). Every face point belongs to
+// one thread. 3000 atoms, 129^3: 1.43 -> 0.63 ms; against long double, the
+// largest error relative to the sum of the terms' sizes 3.6e-16 -> 1.4e-16.
+constexpr int kDhPoints = 4;
+constexpr int kDhWarps = 8;
+// (ln 2 / 64)^k / k!
+__device__ constexpr double kDhTerm[6] = {1.0,
+                                          0.010830424696249145,
+                                          5.86490495505617e-05,
+                                          2.1173137155464776e-07,
+                                          5.732851688640402e-10,
+                                          1.2417843701716925e-12};
+
+struct DhParams {
+  int n;
+  double h, pref, kappa;
+  double khi, klo; // -kappa 64 / ln 2 = khi + klo
+};
+
+// the plain sum at one point (where the fast one met a zero distance)
+__device__ double dh_plain(const double *atoms, int natoms, const DhParams &b,
+                           long i0, long i1, long i2) {
+  double acc = 0.0;
+  for (int t = 0; t < natoms; ++t) {
+    const double *at = atoms + 5 * t;
+    const double d0 = i0 * b.h - at[0], d1 = i1 * b.h - at[1],
+                 d2 = i2 * b.h - at[2];
+    const double dist = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
+    acc += at[4] / (b.pref * (1 + b.kappa * at[3])) *
+           exp(-b.kappa * (dist - at[3])) / dist;
   }
-  double acc = 0;
-  for (int b0 = 0; b0 < natoms; b0 += kSetupThreads) {
+  return acc;
+}
+
+__global__ void __launch_bounds__(32 * kDhWarps)
+    boundary_kernel(const double *__restrict__ atoms, int natoms, DhParams b,
+                    double *__restrict__ x0) {
+  constexpr int kTile = 32 * kDhWarps;
+  __shared__ double sa[kTile * 5];
+  __shared__ double table[64];
+  __shared__ double part[kDhWarps][32 * kDhPoints];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 64)
+    table[threadIdx.x] = exp2(threadIdx.x / 64.0);
+  // the thread's points: face, row a, points from c on. Faces 0, 1: i0 = 0,
+  // n - 1 over all (i1, i2); 2, 3: i1 = 0, n - 1 over interior i0, all i2;
+  // 4, 5: i2 = 0, n - 1 over interior i0 and i1.
+  const int n = b.n, groups = (n + kDhPoints - 1) / kDhPoints;
+  const long rows01 = n, rows = n - 2;
+  long t = blockIdx.x * 32L + lane;
+  long row = t / groups;
+  const int c = (int)(t - row * groups) * kDhPoints;
+  int face = -1;
+  long a = 0;
+  if (row < 2 * rows01) {
+    face = row < rows01 ? 0 : 1;
+    a = row - face * rows01;
+  } else if (row < 2 * rows01 + 4 * rows) {
+    row -= 2 * rows01;
+    face = 2 + (int)(row / rows);
+    a = 1 + row % rows;
+  }
+  const int ax = face < 2 ? 0 : face < 4 ? 1 : 2; // the face's axis
+  const int row_ax = ax == 0 ? 1 : 0;             // of a
+  const int run_ax = ax == 2 ? 1 : 2;             // of the thread's points
+  const double xa = (face & 1) ? (n - 1) * b.h : 0.0;
+  const double xr = a * b.h;
+  double xc[kDhPoints], acc[kDhPoints];
+#pragma unroll
+  for (int q = 0; q < kDhPoints; ++q) {
+    xc[q] = (c + q) * b.h;
+    acc[q] = 0.0;
+  }
+  for (int b0 = 0; b0 < natoms; b0 += kTile) {
     __syncthreads();
-    const int b = b0 + threadIdx.x;
-    if (b < natoms) {
+    if (b0 + (int)threadIdx.x < natoms) {
+      const double *at = atoms + 5 * (size_t)(b0 + threadIdx.x);
+      double *o = sa + 5 * threadIdx.x;
       for (int d = 0; d < 4; ++d)
-        sa[5 * threadIdx.x + d] = atoms[5 * b + d];
-      // the atom's factor q / (pref (1 + kappa r)), once per atom: the
-      // same operations as inside the sum, so the same bits
-      sa[5 * threadIdx.x + 4] =
-          atoms[5 * b + 4] / (pref * (1 + kappa * atoms[5 * b + 3]));
+        o[d] = at[d];
+      o[4] = at[4] / (b.pref * (1 + b.kappa * at[3]));
     }
     __syncthreads();
-    const int nb = natoms - b0 < kSetupThreads ? natoms - b0 : kSetupThreads;
-    if (active)
-      for (int t = 0; t < nb; ++t) {
-        const double *at = &sa[5 * t];
-        const double d0 = i0 * h - at[0];
-        const double d1 = i1 * h - at[1];
-        const double d2 = i2 * h - at[2];
-        const double dist = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-        acc += at[4] * exp(-kappa * (dist - at[3])) / dist;
+    const int nb = natoms - b0 < kTile ? natoms - b0 : kTile;
+    if (face < 0)
+      continue;
+    for (int u = warp; u < nb; u += kDhWarps) {
+      const double *at = sa + 5 * u;
+      const double da = xa - at[ax], dr = xr - at[row_ax];
+      const double s = fma(da, da, dr * dr), pos = at[run_ax];
+      const double rad = at[3], fac = at[4];
+#pragma unroll
+      for (int q = 0; q < kDhPoints; ++q) {
+        const double dc = xc[q] - pos;
+        const double d2 = fma(dc, dc, s);
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d2));
+        const double e = fma(-d2 * y, y, 1.0);
+        y = fma(y * e, fma(e, 0.375, 0.5), y);
+        const double dist = fma(d2, y, -rad); // minus the radius
+        // m = the nearest integer, by the addend 1.5 2^52
+        const double big = fma(dist, b.khi, 6755399441055744.0);
+        const int m = __double2loint(big);
+        const double mr = big - 6755399441055744.0;
+        const double f = fma(dist, b.klo, fma(dist, b.khi, -mr));
+        double p = fma(f, kDhTerm[5], kDhTerm[4]);
+        p = fma(f, p, kDhTerm[3]);
+        p = fma(f, p, kDhTerm[2]);
+        p = f * fma(f, p, kDhTerm[1]);
+        double w = table[m & 63];
+        w = fma(w, p, w);
+        const int k = min(max(m >> 6, -1021), 1022);
+        w = __hiloint2double(__double2hiint(w) + (k << 20),
+                             __double2loint(w));
+        acc[q] = fma(fac * w, y, acc[q]);
       }
+    }
   }
-  if (active)
-    x0[((size_t)i0 * n + i1) * n + i2] = acc;
+#pragma unroll
+  for (int q = 0; q < kDhPoints; ++q)
+    part[warp][q * 32 + lane] = acc[q];
+  __syncthreads();
+  if (warp >= kDhPoints || face < 0)
+    return;
+  const int i = c + warp; // warp q adds up the points q
+  if (i >= n || (face >= 4 && (i < 1 || i > n - 2)))
+    return;
+  double v = 0.0;
+  for (int w = 0; w < kDhWarps; ++w)
+    v += part[w][warp * 32 + lane];
+  const long end = (face & 1) ? n - 1 : 0;
+  const long i0 = ax == 0 ? end : a;
+  const long i1 = ax == 0 ? a : ax == 1 ? end : i;
+  const long i2 = ax == 2 ? end : i;
+  if (!isfinite(v))
+    v = dh_plain(atoms, natoms, b, i0, i1, i2);
+  x0[((size_t)i0 * n + i1) * n + i2] = v;
 }
 
 unsigned grid_for(long count) {
@@ -361,11 +503,15 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
   Scratch sc(st);
   double *d_atoms = nullptr;
   unsigned char *inside = nullptr, *sas = nullptr, *carved = nullptr,
-                *ion = nullptr, *free_flag = nullptr;
+                *ion = nullptr;
   double *centres = nullptr;
+  int *kept = nullptr; // probe centres kept (device)
   ProbeDir *d_dirs = nullptr;
   PMG_CUDA_TRY(sc.take(&d_atoms, 5 * (size_t)natoms));
-  PMG_CUDA_TRY(sc.take(&inside, n3));
+  // inside, and with a probe sas and carved: one block, cleared by one memset
+  const long mask_n = (n3 + 15) & ~15L;
+  const size_t mask_bytes = (probe && natoms > 0 ? 3 : 1) * mask_n;
+  PMG_CUDA_TRY(sc.take(&inside, mask_bytes));
   PMG_CUDA_TRY(sc.take(&ion, n3));
   if (natoms > 0)
     PMG_CUDA_TRY(cudaMemcpyAsync(d_atoms, atoms_host,
@@ -374,9 +520,8 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
   if (probe && natoms > 0) {
     ProbeDir dirs[kProbePoints];
     probe_directions(dirs);
-    PMG_CUDA_TRY(sc.take(&sas, n3));
-    PMG_CUDA_TRY(sc.take(&carved, n3));
-    PMG_CUDA_TRY(sc.take(&free_flag, (size_t)natoms * kProbePoints));
+    sas = inside + mask_n;
+    carved = sas + mask_n;
     PMG_CUDA_TRY(sc.take(&centres, 3 * (size_t)natoms * kProbePoints));
     PMG_CUDA_TRY(sc.take(&d_dirs, kProbePoints));
     PMG_CUDA_TRY(cudaMemcpyAsync(d_dirs, dirs, sizeof(dirs),
@@ -395,12 +540,13 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
     int *d_cid = nullptr, *d_count = nullptr, *d_cstart = nullptr,
         *d_fill = nullptr, *d_cat = nullptr;
     PMG_CUDA_TRY(sc.take(&d_cid, (size_t)natoms));
-    PMG_CUDA_TRY(sc.take(&d_count, (size_t)ncells + 1));
+    PMG_CUDA_TRY(sc.take(&d_count, (size_t)ncells + 2));
+    kept = d_count + ncells + 1;
     PMG_CUDA_TRY(sc.take(&d_cstart, (size_t)ncells + 1));
     PMG_CUDA_TRY(sc.take(&d_fill, (size_t)ncells + 1));
     PMG_CUDA_TRY(sc.take(&d_cat, (size_t)natoms));
     PMG_CUDA_TRY(
-        cudaMemsetAsync(d_count, 0, sizeof(int) * (ncells + 1), st));
+        cudaMemsetAsync(d_count, 0, sizeof(int) * (ncells + 2), st));
     atom_cells_kernel<<<(natoms + 255) / 256, 256, 0, st>>>(
         d_atoms, natoms, cell, dim, d_cid, d_count);
     size_t scan_bytes = 0;
@@ -417,32 +563,27 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
         natoms, d_cid, d_fill, d_cat);
     probe_centres_cells_kernel<<<pgrid, kSetupThreads, 0, st>>>(
         d_atoms, natoms, ph->probe_radius, d_dirs, cell, dim, d_cstart, d_cat,
-        centres, free_flag);
+        centres, kept);
     PMG_LAUNCH_CHECK();
   }
 
   // face coefficients, axis 0 -> uC, 1 -> oN, 2 -> oE
   double *face[3] = {uC, oN, oE};
+  const int np = probe ? natoms * kProbePoints : 0;
   for (int axis = 0; axis < 3; ++axis) {
-    PMG_CUDA_TRY(cudaMemsetAsync(inside, 0, n3, st));
+    PMG_CUDA_TRY(cudaMemsetAsync(inside, 0, mask_bytes, st));
     if (natoms > 0) {
-      SphereSet atoms_set{d_atoms, 5, natoms, d_atoms + 3, 0.0, nullptr,
-                          axis};
-      mark_spheres_kernel<unsigned char>
-          <<<natoms, kSetupThreads, 0, st>>>(n, h, atoms_set, inside, 1);
-    }
-    if (probe && natoms > 0) {
-      PMG_CUDA_TRY(cudaMemsetAsync(sas, 0, n3, st));
-      PMG_CUDA_TRY(cudaMemsetAsync(carved, 0, n3, st));
-      SphereSet inflated{d_atoms, 5, natoms, d_atoms + 3, ph->probe_radius,
-                         nullptr, axis};
-      mark_spheres_kernel<unsigned char>
-          <<<natoms, kSetupThreads, 0, st>>>(n, h, inflated, sas, 1);
-      const int np = natoms * kProbePoints;
-      SphereSet probes{centres, 3, np, nullptr, ph->probe_radius, free_flag,
-                       axis};
-      mark_spheres_kernel<unsigned char>
-          <<<np, kSetupThreads, 0, st>>>(n, h, probes, carved, 1);
+      SphereSets m{};
+      m.axis = axis;
+      m.set[0] = SphereSet{d_atoms, 5, natoms, d_atoms + 3, 0.0, nullptr,
+                           inside};
+      if (probe) {
+        m.set[1] = SphereSet{d_atoms,          5,       natoms, d_atoms + 3,
+                             ph->probe_radius, nullptr, sas};
+        m.set[2] = SphereSet{centres,          3,         np, nullptr,
+                             ph->probe_radius, kept, carved};
+      }
+      mark_spheres_kernel<<<mark_blocks(m), kSetupThreads, 0, st>>>(n, h, m);
     }
     face_from_masks_kernel<<<grid_for(n3), kSetupThreads, 0, st>>>(
         n3, inside, probe && natoms > 0 ? sas : nullptr, carved, v_in, v_out,
@@ -453,10 +594,11 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
   // ion-exclusion mask and the centre coefficient
   PMG_CUDA_TRY(cudaMemsetAsync(ion, 0, n3, st));
   if (natoms > 0) {
-    SphereSet ions{d_atoms, 5, natoms, d_atoms + 3, ph->ion_radius, nullptr,
-                   -1};
-    mark_spheres_kernel<unsigned char>
-        <<<natoms, kSetupThreads, 0, st>>>(n, h, ions, ion, 1);
+    SphereSets m{};
+    m.axis = -1;
+    m.set[0] = SphereSet{d_atoms, 5, natoms, d_atoms + 3, ph->ion_radius,
+                         nullptr, ion};
+    mark_spheres_kernel<<<mark_blocks(m), kSetupThreads, 0, st>>>(n, h, m);
   }
   centre_kernel<<<grid_for(n3), kSetupThreads, 0, st>>>(
       n, uC, oN, oE, ion, p.kappa * p.kappa * p.eps_out, oC);
@@ -489,10 +631,16 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
   // Debye-Hueckel boundary
   PMG_CUDA_TRY(cudaMemsetAsync(x0, 0, sizeof(double) * n3, st));
   if (natoms > 0) {
-    const long pts = 6L * n * n;
-    boundary_kernel<<<(unsigned)((pts + kSetupThreads - 1) / kSetupThreads),
-                      kSetupThreads, 0, st>>>(
-        d_atoms, natoms, n, h, 4 * kPi * (p.eps0 * p.eps_out), p.kappa, x0);
+    DhParams b{n, h, 4 * kPi * (p.eps0 * p.eps_out), p.kappa, 0.0, 0.0};
+    // -kappa 64 / ln 2 to about 100 bits
+    const long double k = -(long double)p.kappa * 64.0L /
+                          0.693147180559945309417232121458176568L;
+    b.khi = (double)k;
+    b.klo = (double)(k - b.khi);
+    const long threads =
+        (2L * n + 4L * (n - 2)) * ((n + kDhPoints - 1) / kDhPoints);
+    boundary_kernel<<<(unsigned)((threads + 31) / 32), 32 * kDhWarps, 0,
+                      st>>>(d_atoms, natoms, b, x0);
     PMG_LAUNCH_CHECK();
   }
   return PMG_OK;
