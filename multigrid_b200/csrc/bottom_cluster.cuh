@@ -108,22 +108,6 @@ __device__ __forceinline__ SplitPoint<ROW, PLANE> split_point(int i, int j,
                                 o + split_entry<ODD>(i + 1)};
 }
 
-// s / c from y, the reciprocal of c rounded to nearest: two residual
-// corrections of the product s y. The first leaves q within an ulp of the
-// quotient, so the second gives it correctly rounded (Markstein, IBM J. Res.
-// Dev. 34, 1990), the bits of the divide, in five dependent operations (a
-// double divide is ~110 cycles, these ~40).
-__device__ __forceinline__ double div_by_recip(double s, double c, double y) {
-  double q = s * y;
-  q = __fma_rn(__fma_rn(-q, c, s), y, q);
-  return __fma_rn(__fma_rn(-q, c, s), y, q);
-}
-__device__ __forceinline__ float div_by_recip(float s, float c, float y) {
-  float q = s * y;
-  q = __fmaf_rn(__fmaf_rn(-q, c, s), y, q);
-  return __fmaf_rn(__fmaf_rn(-q, c, s), y, q);
-}
-
 // Level 1 with at most kInvMax unknowns (7^3 points and fewer; the
 // refinement paths): the inverse of its interior operator, dense, computed
 // when the hierarchy is built. The CG it replaces there runs 11 to 20

@@ -26,13 +26,17 @@
 // double; the pass is bound more by instruction issue than by the copies). Plane k is computed
 // from the stages of k - 1, k and k + 1 while the next S - 3 planes are in
 // flight, so the bytes in flight are set by the ring, not by registers.
-// A warp computes a row: each lane four consecutive points from 16-byte
-// shared-memory loads, the one west or east neighbour outside its four by a
-// shuffle, and stores the four results with one 16-byte store. A point's
-// seven coefficients come from a 128-entry table in shared memory indexed
-// by its code byte (two 16-byte loads instead of six bit tests and
-// selects and a table lookup). The arithmetic is gs7_code_color_kernel's,
-// term for term, so the bits are the same.
+// A warp computes a row, one point per lane. A point's seven coefficients and
+// the reciprocal of its divisor come from a 128-entry table in shared memory
+// indexed by its code byte (wide loads instead of six bit tests and selects
+// and a table lookup). The arithmetic is gs7_code_color_kernel's, term for
+// term, the divide as two corrections of the product with the reciprocal
+// (div_by_recip: the same bits), so the bits are the same. Before, a lane took
+// four consecutive points by 16-byte loads: rows of 33, 65 and 129 points
+// then need a round more than a multiple of 32 lanes (9, 17 and 33 quads),
+// and in double 96 registers left two CTAs per SM, with the IEEE divide in
+// every point. Per pass, float: 65^3 4.7 -> @@, 129^3 9.3 -> @@, 257^3 29.9 ->
+// @@ us; double: 129^3 21.9 -> @@, 161^3 32.8 -> @@ us.
 //
 // A pass reads only the other colour of x and writes only its own, so the
 // stages never hold values the pass changes. Rows and planes outside the
@@ -51,6 +55,7 @@
 #include <type_traits>
 
 #include "gs27_tma.cuh"
+#include "row_stencil.cuh"
 #include "split_layout.cuh"
 
 namespace pmg {
@@ -63,7 +68,7 @@ template <typename T> struct StreamCfg {
   static constexpr int THREADS = 32 * (J + 1);
   // CTAs per SM the ring's shared memory allows at 257^3 (registers capped
   // to match)
-  static constexpr int MIN_CTAS = sizeof(T) == 4 ? 3 : 2;
+  static constexpr int MIN_CTAS = 3;
 };
 
 // Tensor maps of the colour-split x, f (element type T) and code bytes of a
@@ -143,35 +148,18 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
                    smem_addr(bar))
                : "memory");
 }
-
-// num / (c + 0), rounded to T, with c the divisor of table entry b.
-// Double: IEEE division. Float: num times the double reciprocal of the
-// divisor, rounded to float. That product is within 2^-51 (relative) of
-// num / c (two double roundings), while a quotient of two 24-bit floats
-// that is not itself a float lies at least 2^-49 (relative) from every
-// rounding midpoint between floats ((a - c m) is a nonzero multiple of the
-// smallest exponent's unit), so both round to the same float: the bits of
-// the division, without its special-case branch. Quotients that are
-// floats, zeros, infinities and NaNs come out the same too.
-__device__ __forceinline__ double div_by_table(double num, double c,
-                                               const double *, unsigned) {
-  return num / (c + 0.0);
-}
-__device__ __forceinline__ float div_by_table(float num, float,
-                                              const double *rtab,
-                                              unsigned b) {
-  return (float)((double)num * rtab[b]);
+// the same in the threads with `on`, without a branch (mbar.cuh, send)
+__device__ __forceinline__ void mbar_arrive_if(bool on, uint64_t *bar) {
+  asm volatile("{\n"
+               ".reg .pred p;\n"
+               "setp.ne.u32 p, %1, 0;\n"
+               "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n"
+               "}\n" ::"r"(smem_addr(bar)),
+               "r"((unsigned)on)
+               : "memory");
 }
 
-// a row parity given at compile time (std::true_type / std::false_type) or
-// at run time (bool)
-__device__ __forceinline__ bool row_parity(bool b) { return b; }
-template <bool B>
-__device__ __forceinline__ bool row_parity(std::integral_constant<bool, B>) {
-  return B;
-}
-
-// four consecutive entries
+// half of a coefficient table row
 template <typename T> struct alignas(16) Quad {
   T x, y, z, w;
 };
@@ -193,11 +181,9 @@ __global__ void __launch_bounds__(StreamCfg<T>::THREADS,
   using V = Quad<T>;
   extern __shared__ __align__(128) unsigned char sm[];
   // per code byte (its low seven bits) the point's seven coefficients in
-  // the order the update uses them: n, s, e, w, down, up, oC (one spare)
+  // the order the update uses them: n, s, e, w, down, up, oC, and the
+  // reciprocal of oC (div_by_recip: the bits of the divide by oC + 0)
   __shared__ __align__(16) T ctab[128][8];
-  // float: the double reciprocal of each code's divisor oC + 0 (see
-  // div_by_table)
-  __shared__ double rtab[sizeof(T) == 4 ? 128 : 1];
   // full[s]: the slot's boxes landed (the producer's arrival and their
   // bytes); empty[s]: every consumer warp is done with it
   uint64_t *full = reinterpret_cast<uint64_t *>(sm + S * sh.slot);
@@ -232,9 +218,7 @@ __global__ void __launch_bounds__(StreamCfg<T>::THREADS,
     t[4] = (b & 32u) ? L.uh : L.ul;
     t[5] = (b & 16u) ? L.uh : L.ul;
     t[6] = octab[b];
-    t[7] = T(0);
-    if constexpr (sizeof(T) == 4)
-      rtab[b] = 1.0 / (double)(t[6] + T(0));
+    t[7] = T(1) / t[6];
   }
   __syncthreads();
   auto slot_of = [&](int kk) { return (kk - kfirst) % S; };
@@ -314,122 +298,50 @@ __global__ void __launch_bounds__(StreamCfg<T>::THREADS,
       // pass's colour) or 2 + 2e; interior e in [elo, ehi]. West and east
       // are entries e - 1, e (odd i) or e, e + 1 (even i) of the other half.
       const long row = (long)sp.row(j, k) + want * sp.hp;
-      // the row's parity is the same for the whole warp. Float: each case
-      // compiled on its own, so the per-point selects between them fold away
-      // (1-2% per pass at 257^3); double keeps one body, whose two copies
-      // would spill (258 against 254 us per four passes)
-      auto row_pass = [&](auto odd_c) {
-        const bool odd = row_parity(odd_c);
-        const int elo = odd ? 1 : 0;
-        const int ehi = odd ? (d.nx - 2) / 2 : (d.nx - 3) / 2;
-        // every lane takes part in each round (the shuffles); lane g of the
-        // round takes entries 4g .. 4g + 3
-        for (int g0 = 0; 4 * g0 <= ehi; g0 += 32) {
-          const int g = g0 + lane, e4 = 4 * g;
-          const bool act = e4 <= ehi;
-          V vn{}, vs{}, vu{}, vd{}, vo{}, vf{};
-          unsigned cb = 0;
-          if (act) {
-            vn = *reinterpret_cast<const V *>(xn + e4);
-            vs = *reinterpret_cast<const V *>(xs + e4);
-            vu = *reinterpret_cast<const V *>(xu + e4);
-            vd = *reinterpret_cast<const V *>(xd + e4);
-            vo = *reinterpret_cast<const V *>(xo + e4);
-            vf = *reinterpret_cast<const V *>(fr + e4);
-            cb = *reinterpret_cast<const unsigned *>(cr + e4);
-          }
-          // the other-half entry just outside the four: e4 - 1 (odd i, the
-          // previous lane's last) or e4 + 4 (even i, the next lane's first);
-          // read directly where that lane is in another round or idle
-          const T up = __shfl_up_sync(0xffffffffu, vo.w, 1);
-          const T down = __shfl_down_sync(0xffffffffu, vo.x, 1);
-          T edge = odd ? up : down;
-          if (act && odd && lane == 0 && e4 > 0)
-            edge = xo[e4 - 1];
-          if (act && !odd && (lane == 31 || e4 + 4 > ehi))
-            edge = xo[e4 + 4];
-          const T xw[4] = {odd ? edge : vo.x, odd ? vo.x : vo.y,
-                           odd ? vo.y : vo.z, odd ? vo.z : vo.w};
-          const T xe[4] = {odd ? vo.x : vo.y, odd ? vo.y : vo.z,
-                           odd ? vo.z : vo.w, odd ? vo.w : edge};
-          const T an[4] = {vn.x, vn.y, vn.z, vn.w};
-          const T as[4] = {vs.x, vs.y, vs.z, vs.w};
-          const T au[4] = {vu.x, vu.y, vu.z, vu.w};
-          const T ad[4] = {vd.x, vd.y, vd.z, vd.w};
-          const T af[4] = {vf.x, vf.y, vf.z, vf.w};
-          T out[4];
-          if (oc_coded) {
-            // every coefficient from the code byte's table entry (the same
-            // values gs7_code_color_kernel selects); points outside the row's
-            // interior compute from table entries too and are not stored
-  #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-              const T *t = ctab[(cb >> (8 * m)) & 127u];
-              const Quad<T> c0 = *reinterpret_cast<const Quad<T> *>(t);
-              const Quad<T> c1 = *reinterpret_cast<const Quad<T> *>(t + 4);
-              const T sum = c0.x * an[m] + c0.y * as[m] + c0.z * xe[m] +
-                            c0.w * xw[m] + c1.x * ad[m] + c1.y * au[m];
-              out[m] = div_by_table(KEEP ? af[m] + sum : af[m] + T(0) * sum,
-                                    c1.z, rtab,
-                                    (cb >> (8 * m)) & 127u);
-            }
+      // one point per lane and round: consecutive lanes read consecutive
+      // entries, and a row of 64 or 128 points is whole rounds
+      const bool odd = ((1 + j + k) & 1) == want;
+      const int elo = odd ? 1 : 0;
+      const int ehi = odd ? (d.nx - 2) / 2 : (d.nx - 3) / 2;
+      const T *west = xo - (odd ? 1 : 0), *east = west + 1;
+      T *dst = x + row;
+#pragma unroll (sizeof(T) == 4 ? 2 : 1)
+      for (int e = elo + lane; e <= ehi; e += 32) {
+        const unsigned b = cr[e];
+        const T vn = xn[e], vs = xs[e], ve = east[e], vw = west[e],
+                vd = xd[e], vu = xu[e], vf = fr[e];
+        T sum, q;
+        if (oc_coded) {
+          const T *t = ctab[b & 127u];
+          const Quad<T> c0 = *reinterpret_cast<const Quad<T> *>(t);
+          const Quad<T> c1 = *reinterpret_cast<const Quad<T> *>(t + 4);
+          sum = c0.x * vn + c0.y * vs + c0.z * ve + c0.w * vw +
+                c1.x * vd + c1.y * vu;
+          q = div_by_recip(KEEP ? vf + sum : vf + T(0) * sum, c1.z, c1.w);
+        } else {
+          const int p = (int)(row + e);
+          Couplings<T> cp{};
+          if (coded) {
+            cp.e = (b & 1u) ? L.eh : L.el;
+            cp.w = (b & 2u) ? L.eh : L.el;
+            cp.n = (b & 4u) ? L.nh : L.nl;
+            cp.s = (b & 8u) ? L.nh : L.nl;
+            cp.u = (b & 16u) ? L.uh : L.ul;
+            cp.dn = (b & 32u) ? L.uh : L.ul;
           } else {
-  #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-              const int e = e4 + m;
-              const bool in = act && e >= elo && e <= ehi;
-              const unsigned b = (cb >> (8 * m)) & 0xffu;
-              const int p = (int)(row + e);
-              Couplings<T> cp{};
-              if (coded) {
-                cp.e = (b & 1u) ? L.eh : L.el;
-                cp.w = (b & 2u) ? L.eh : L.el;
-                cp.n = (b & 4u) ? L.nh : L.nl;
-                cp.s = (b & 8u) ? L.nh : L.nl;
-                cp.u = (b & 16u) ? L.uh : L.ul;
-                cp.dn = (b & 32u) ? L.uh : L.ul;
-              } else if (in) {
-                cp = array_couplings<T>(oE, oN, uC, p,
-                                        split_nb(sp, p, odd ? 1 : 2, want));
-              }
-              const T sum = cp.n * an[m] + cp.s * as[m] + cp.e * xe[m] +
-                            cp.w * xw[m] + cp.dn * ad[m] + cp.u * au[m];
-              const T c = in ? oC[p] : T(1);
-              out[m] = (KEEP ? af[m] + sum : af[m] + T(0) * sum) / (c + T(0));
-            }
+            cp = array_couplings<T>(oE, oN, uC, p,
+                                    split_nb(sp, p, odd ? 1 : 2, want));
           }
-          if (act) {
-            T *dst = x + row + e4;
-            if (e4 >= elo && e4 + 3 <= ehi) {
-              V v;
-              v.x = out[0];
-              v.y = out[1];
-              v.z = out[2];
-              v.w = out[3];
-              *reinterpret_cast<V *>(dst) = v;
-            } else {
-  #pragma unroll
-              for (int m = 0; m < 4; ++m)
-                if (e4 + m >= elo && e4 + m <= ehi)
-                  dst[m] = out[m];
-            }
-          }
+          sum = cp.n * vn + cp.s * vs + cp.e * ve + cp.w * vw + cp.dn * vd +
+                cp.u * vu;
+          q = (KEEP ? vf + sum : vf + T(0) * sum) / (oC[p] + T(0));
         }
-      };
-      const bool row_odd = ((1 + j + k) & 1) == want;
-      if constexpr (sizeof(T) == 4) {
-        if (row_odd)
-          row_pass(std::true_type{});
-        else
-          row_pass(std::false_type{});
-      } else {
-        row_pass(row_odd);
+        dst[e] = q;
       }
     }
     // plane k - 1 is no longer needed by this warp
     __syncwarp();
-    if (lane == 0)
-      mbar_arrive(&empty[slot_of(k - 1)]);
+    mbar_arrive_if(lane == 0, &empty[slot_of(k - 1)]);
   }
 }
 
