@@ -114,3 +114,46 @@ def test_low_levels_of_the_cycle(restatement, base, nlev):
         assert np.linalg.norm(x - xo) <= tol * np.linalg.norm(xo), prec
         if prec == "fp64":
             assert r.cycles == co
+
+
+def band(n, m, seed):
+    """LINPACK upper band storage of a symmetric positive definite matrix
+    (diagonally dominant), column-major with lda = m + 1."""
+    rng = np.random.default_rng(seed)
+    a = np.zeros((n, m + 1))  # row j: column j of the band
+    for j in range(n):
+        k0 = max(0, m - j)
+        a[j, k0:m] = rng.uniform(-1.0, 0.0, m - k0)
+    a[:, m] = 2.0 * m + rng.uniform(1.0, 2.0, n)
+    return a.ravel()
+
+
+# one unknown; half widths 0, around LINPACK's unrolling by five and at a
+# warp; a 9^3 level's 27-point band; one that does not fit on chip
+@pytest.mark.parametrize("n,m", [(1, 0), (4, 0), (6, 1), (27, 13), (40, 31),
+                                 (60, 17), (343, 57), (400, 100)])
+def test_band_sizes_bit_for_bit(restatement, n, m):
+    a = band(n, m, n + m)
+    want = a.copy()
+    assert restatement.dpbfa(want, m + 1, n, m) == 0
+    g = T(a)
+    assert pmgc.Vdpbfa(g, m + 1, n, m) == 0
+    assert np.array_equal(g.cpu().numpy(), want)
+    b = np.random.default_rng(m).normal(size=n)
+    xo = b.copy()
+    restatement.dpbsl(want, m + 1, n, m, xo)
+    x = T(b)
+    pmgc.Vdpbsl(g, m + 1, n, m, x)
+    assert np.array_equal(x.cpu().numpy(), xo)
+
+
+@pytest.mark.parametrize("bad", [1, 5, 27])
+def test_band_bad_pivot_leaves_later_columns(restatement, bad):
+    n, m = 27, 13
+    a = band(n, m, 3)
+    a[(bad - 1) * (m + 1) + m] = -1.0
+    want = a.copy()
+    assert restatement.dpbfa(want, m + 1, n, m) == bad
+    g = T(a)
+    assert pmgc.Vdpbfa(g, m + 1, n, m) == bad
+    assert np.array_equal(g.cpu().numpy(), want)
