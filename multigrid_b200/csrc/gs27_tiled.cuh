@@ -134,6 +134,69 @@ __device__ __forceinline__ void gs27_step_at(const Dims &d, const Op14<T> &A,
   }
 }
 
+// One sub-colour step's point of a thread, for tiles with at most one.
+template <int TT, int W, int H> struct Gs27Slot {
+  static constexpr int NU = TT / 2 + H;
+  static_assert(NU * NU <= Gs27Tile<TT>::THREADS, "one point per thread");
+  bool ok;
+  int sidx, p;
+  __device__ __forceinline__ Gs27Slot(const Dims &d, int ti0, int tj0, int k,
+                                      int order) {
+    const int s = (order >> (2 * (3 - H))) & 3;
+    const int pi = s & 1, pj = s >> 1;
+    const int v = threadIdx.x / NU, u = threadIdx.x - v * NU;
+    const int i = ti0 - H + ((pi - (ti0 - H)) & 1) + 2 * u;
+    const int j = tj0 - H + ((pj - (tj0 - H)) & 1) + 2 * v;
+    ok = v < NU && i >= 2 && i <= d.nx - 1 && j >= 2 && j <= d.ny - 1;
+    sidx = (i - (ti0 - kH27)) + W * (j - (tj0 - kH27));
+    p = ok ? d.at(i, j, k) : 0;
+  }
+};
+
+// The four steps on tiles of 8 and 16, where every thread has at most one
+// point per step: each step's couplings are loaded two steps ahead, before a
+// barrier that their use follows. A step that loads where it uses them waits
+// out a global load's latency (in several batches: the compiler kept 32
+// registers and sank the loads to their uses), four times in a row, which was
+// most of a small level's launch. Tiles of 32 hold several points a thread and
+// have the warps to hide that latency. ready(): called once the first two
+// steps' loads are in flight; returns when the staged x may be read. Per
+// launch: float 33^3 by TMA 4.8 -> 3.7 us, 65^3 7.6 -> 7.5; in
+// gs27_phase_kernel 33^3-49^3 float 5.4 -> 4.5, double 6.2 -> 5.4.
+template <typename T, int TT, int W, int PS, class Ready>
+__device__ __forceinline__ void gs27_steps(const Dims &d, const Op14<T> &A,
+                                           const T *cc, const T *fc, T *xk,
+                                           int ti0, int tj0, int k, int order,
+                                           Ready ready) {
+  const int sy = d.sy(), sz = d.sz();
+  const Gs27Slot<TT, W, 3> s3(d, ti0, tj0, k, order);
+  const Gs27Slot<TT, W, 2> s2(d, ti0, tj0, k, order);
+  const Gs27Slot<TT, W, 1> s1(d, ti0, tj0, k, order);
+  const Gs27Slot<TT, W, 0> s0(d, ti0, tj0, k, order);
+  Gs27Point<T> a, b;
+  auto load = [&](bool ok, int p, Gs27Point<T> &c) {
+    if (ok)
+      gs27_load(A, cc, fc, p, sy, sz, c);
+  };
+  auto update = [&](bool ok, int q, const Gs27Point<T> &c) {
+    if (ok)
+      xk[q] = gs27_update<T, W>(c, &xk[q], &xk[q - PS], &xk[q + PS]);
+  };
+  load(s3.ok, s3.p, a);
+  load(s2.ok, s2.p, b);
+  ready();
+  update(s3.ok, s3.sidx, a);
+  load(s1.ok, s1.p, a);
+  __syncthreads();
+  update(s2.ok, s2.sidx, b);
+  load(s0.ok, s0.p, b);
+  __syncthreads();
+  update(s1.ok, s1.sidx, a);
+  __syncthreads();
+  update(s0.ok, s0.sidx, b);
+  __syncthreads();
+}
+
 // gs27_step_at on the staged planes of gs27_phase_kernel (W x W each, plane
 // k - 1 first)
 template <typename T, int TT, int H>
@@ -170,16 +233,24 @@ __global__ void __launch_bounds__(Gs27Tile<TT>::THREADS)
     const T *src = (pl == 1 ? own : nb) + (in ? d.at(i, j, k - 1 + pl) : 0);
     cp_async_zfill<sizeof(T)>(&xs[q], src, in);
   }
-  cp_async_wait_all();
-  __syncthreads();
-  gs27_step<T, TT, 3>(d, A, cc, fc, xs, ti0, tj0, k, order);
-  __syncthreads();
-  gs27_step<T, TT, 2>(d, A, cc, fc, xs, ti0, tj0, k, order);
-  __syncthreads();
-  gs27_step<T, TT, 1>(d, A, cc, fc, xs, ti0, tj0, k, order);
-  __syncthreads();
-  gs27_step<T, TT, 0>(d, A, cc, fc, xs, ti0, tj0, k, order);
-  __syncthreads();
+  if constexpr (TT <= 16) {
+    gs27_steps<T, TT, W, W * W>(d, A, cc, fc, xs + W * W, ti0, tj0, k, order,
+                                [] {
+                                  cp_async_wait_all();
+                                  __syncthreads();
+                                });
+  } else {
+    cp_async_wait_all();
+    __syncthreads();
+    gs27_step<T, TT, 3>(d, A, cc, fc, xs, ti0, tj0, k, order);
+    __syncthreads();
+    gs27_step<T, TT, 2>(d, A, cc, fc, xs, ti0, tj0, k, order);
+    __syncthreads();
+    gs27_step<T, TT, 1>(d, A, cc, fc, xs, ti0, tj0, k, order);
+    __syncthreads();
+    gs27_step<T, TT, 0>(d, A, cc, fc, xs, ti0, tj0, k, order);
+    __syncthreads();
+  }
 
   // write the tile's interior points of plane k
   const int i_max = d.nx - 1, j_max = d.ny - 1;

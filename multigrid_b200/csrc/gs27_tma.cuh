@@ -317,8 +317,7 @@ __global__ void __launch_bounds__(Gs27Tile<TT>::THREADS, 2048 /
 // against 13.9 us per launch at 65^3, 8.1 against 9.5 at 33^3). err and
 // extra_tx as gs27_tma_kernel's.
 template <int TT>
-__global__ void __launch_bounds__(Gs27Tile<TT>::THREADS, 2048 /
-                                  Gs27Tile<TT>::THREADS)
+__global__ void __launch_bounds__(Gs27Tile<TT>::THREADS)
     gs27_tma_square_kernel(const __grid_constant__ Gs27TmaMaps maps, Dims d,
                            Op14<float> A, const float *__restrict__ fc,
                            float *out, int kfirst, int order, int *err,
@@ -343,29 +342,22 @@ __global__ void __launch_bounds__(Gs27Tile<TT>::THREADS, 2048 /
     tma_load_3d(xs + kBox, &maps.own, cx, cy, z, &bar);
     tma_load_3d(xs + 2 * kBox, &maps.nb, cx, cy, z + 1, &bar);
   }
-  const bool ok = mbar_wait(&bar, 0);
-  if (__syncthreads_or(!ok)) {
+  // box column c holds 1-based i = ti0 - 5 + c, row r holds j = tj0 - 4 + r;
+  // the steps' origin is (ti0 - 4, tj0 - 4): one column on
+  float *xc = xs + kBox + 1;
+  bool lost = false;
+  gs27_steps<float, TT, W, kBox>(d, A, nullptr, fc, xc, ti0, tj0, k, order,
+                                 [&] {
+                                   lost = __syncthreads_or(
+                                       !mbar_wait(&bar, 0));
+                                 });
+  if (lost) { // (block-uniform; the tile's values are not stored)
     if (threadIdx.x == 0) {
       atomicOr(err, 1);
       (void)mbar_wait(&bar, 0); // the copies land before the block leaves
     }
     return;
   }
-  // box column c holds 1-based i = ti0 - 5 + c, row r holds j = tj0 - 4 + r;
-  // gs27_step_at's origin is (ti0 - 4, tj0 - 4): one column on
-  float *xc = xs + kBox + 1;
-  gs27_step_at<float, TT, W, kBox, 3>(d, A, nullptr, fc, xc, ti0, tj0, k,
-                                      order);
-  __syncthreads();
-  gs27_step_at<float, TT, W, kBox, 2>(d, A, nullptr, fc, xc, ti0, tj0, k,
-                                      order);
-  __syncthreads();
-  gs27_step_at<float, TT, W, kBox, 1>(d, A, nullptr, fc, xc, ti0, tj0, k,
-                                      order);
-  __syncthreads();
-  gs27_step_at<float, TT, W, kBox, 0>(d, A, nullptr, fc, xc, ti0, tj0, k,
-                                      order);
-  __syncthreads();
   const int i_max = d.nx - 1, j_max = d.ny - 1;
 #pragma unroll
   for (int m = 0; m < (TT * TT + NT - 1) / NT; ++m) {
