@@ -486,8 +486,8 @@ int pmg_setup_fine(int n, double h, const double *atoms, int natoms,
  * stream-ordered on `stream` (scratch from the stream-ordered allocator);
  * atoms are host rows, validated like pmg_setup_fine. oE oN uC oC and f are
  * bit-identical to pmg_setup_fine (same marking bounds and sums, charges
- * summed per grid point in atom order); x0 uses CUDA's exp and agrees to a
- * few ulp. */
+ * summed per grid point in atom order); x0 uses its own exponential and
+ * reciprocal square root and agrees to a few ulp. */
 int pmg_setup_fine_d(int n, double h, const double *atoms, int natoms,
                      const pmg_physics *phys, double *oC, double *oE,
                      double *oN, double *uC, double *f, double *x0,
@@ -653,7 +653,9 @@ int pmg_get_level(pmg_problem *p, int level, double *dst);
 
 /* Mixed precision: relative residual reduction at which the coarsest-level
  * CG stops on each correction (default 1e-4; the FP64 path always runs the
- * class's absolute 1e-8 test). */
+ * class's absolute 1e-8 test). A coarsest level of at most 125 unknowns is
+ * solved by its inverse on the refinement paths; there the setting is kept
+ * but changes nothing unless a pivot fails and the CG runs. */
 int pmg_problem_set_coarse_rtol(pmg_problem *p, double rtol);
 
 /* on != 0: pmg_solve drives its cycles from the host (one cycle-graph
