@@ -554,6 +554,13 @@ int pmg_set_finest_streaming(int on);
  * with: use new problems on both sides of the switch. */
 int pmg_test_tma_short_delivery(int bytes);
 
+/* For testing the order of the messages in the one-launch lowest levels: in
+ * solves launched or captured afterwards the warps without a grid point
+ * start their last wait of the downward half `us` microseconds late (0 to
+ * 10000, 0 restores). Changes no result. A captured solve graph keeps the
+ * value it was captured with. */
+int pmg_test_idle_warp_delay(int us);
+
 /* Creates a problem on the current CUDA device; allocates its hierarchy.
  * stream may be NULL (a private stream is created). */
 int pmg_problem_create(int base, int nlev, double box, int precision,

@@ -26,7 +26,13 @@
 // an odd plane for its even ones, so a sender can be at most one phase ahead
 // of a receiver and only after the receiver has all bytes of its own phase
 // (an even plane's interpolated values are not sent: its odd neighbours read
-// it only after its next sweep).
+// it only after its next sweep). A wait must also be over in every warp of
+// the plane before the plane sends what the mbarrier's next phase depends on:
+// a warp that polls only after that phase has completed too sees the parity
+// it waits for as not yet reached. In a sweep the colours' barriers see to
+// that; the wait before the defect has a barrier of its own, because a warp
+// without a point (every other one where the top level has at most 9 points
+// per axis) sends nothing that would hold the others back.
 // Measured per cycle: 105 us (levels 5^3, 9^3, 17^3 of a 257^3 mixed solve) ->
 // 35 us, 90 -> 27 us at 65^3; in double, where these levels were 31 launches,
 // 250 -> 46 us (129^3). The same kernel serves many concurrent solves: one CTA
@@ -75,6 +81,9 @@ template <typename T> struct BottomArgs {
   // and whether it may be used
   const double *inv;
   const int *inv_ok;
+  // a test's delay of the warps without a point before they wait for the
+  // values that the defect reads, in units of 16 us (0: none)
+  int idle_delay;
 };
 
 constexpr int kBcThreads = 512;
@@ -645,13 +654,19 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
         T ax = T(0);
 #pragma unroll 1
         for (int s = 0; s < 3; ++s) {
+          if (s == 2 && a.idle_delay && !__any_sync(0xffffffffu, own))
+            for (int q16 = 0; q16 < a.idle_delay; ++q16)
+              __nanosleep(16384);
           if (s == 2 ? g == 0 : g == 1 || s > 0 || phase == 1) {
             lost |= !mbar_wait_cluster(&sm.bar_x[g], x_parity);
             x_parity ^= 1u;
             mbar_expect_tx_if(first, &sm.bar_x[g], x_bytes);
           }
-          if (s == 2)
+          if (s == 2) {
+            if (g == 0)
+              group_barrier(); // every warp has seen that phase
             break;
+          }
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             if ((colour & 3) == c) { // whole warps (no point: zeros)

@@ -261,6 +261,8 @@ bool tma_disabled() { return g_tma_on.load() == 0; }
 std::atomic<int> g_stream_on{1};
 // pmg_test_tma_short_delivery: extra bytes every stage waits for
 std::atomic<unsigned> g_tma_extra_tx{0};
+// pmg_test_idle_warp_delay, in units of 16 us
+std::atomic<int> g_idle_delay{0};
 
 int level_n(int base, int L) { return base * (1 << L) + 1; }
 
@@ -564,6 +566,7 @@ template <typename T> BottomArgs<T> bottom_args(pmg_problem *p, int top) {
   a.kernel_err = p->kernel_err;
   a.inv = p->inv1;
   a.inv_ok = p->inv1_ok;
+  a.idle_delay = g_idle_delay.load();
   return a;
 }
 
@@ -1690,6 +1693,15 @@ int pmg_test_tma_short_delivery(int bytes) {
     return PMG_ERR_ARG;
   }
   g_tma_extra_tx.store((unsigned)bytes);
+  return PMG_OK;
+}
+
+int pmg_test_idle_warp_delay(int us) {
+  if (us < 0 || us > 10000) {
+    set_last_message("pmg_test_idle_warp_delay: us must be in [0, 10000]");
+    return PMG_ERR_ARG;
+  }
+  g_idle_delay.store((us + 15) / 16);
   return PMG_OK;
 }
 
