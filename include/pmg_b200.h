@@ -554,6 +554,12 @@ int pmg_set_finest_streaming(int on);
  * with: use new problems on both sides of the switch. */
 int pmg_test_tma_short_delivery(int bytes);
 
+/* The same for the messages between the CTAs of the kernels that hold the
+ * lowest levels on chip (the coarsest CG above 9^3, Vcghs above 9^3, the
+ * one-launch lowest levels): every wait expects `bytes` (a multiple of 16 up
+ * to 2^16, 0 restores) more than arrive. */
+int pmg_test_message_short_delivery(int bytes);
+
 /* For testing the order of the messages in the one-launch lowest levels: in
  * solves launched or captured afterwards the warps without a grid point
  * start their last wait of the downward half `us` microseconds late (0 to

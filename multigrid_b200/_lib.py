@@ -125,6 +125,7 @@ _sig("pmg_set_tma_staging", c_int, c_int)
 _sig("pmg_set_finest_streaming", c_int, c_int)
 _sig("pmg_test_tma_short_delivery", c_int, c_int)
 _sig("pmg_test_idle_warp_delay", c_int, c_int)
+_sig("pmg_test_message_short_delivery", c_int, c_int)
 _sig("pmg_problem_set_coded_couplings", c_int, _V, c_int)
 _sig("pmg_problem_coded_couplings", c_int, _V, PI)
 _sig("pmg_problem_finest_streamed", c_int, _V, PI)

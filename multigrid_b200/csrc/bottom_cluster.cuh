@@ -84,6 +84,7 @@ template <typename T> struct BottomArgs {
   // a test's delay of the warps without a point before they wait for the
   // values that the defect reads, in units of 16 us (0: none)
   int idle_delay;
+  unsigned extra_tx; // a test's bytes that no message brings (0)
 };
 
 constexpr int kBcThreads = 512;
@@ -544,7 +545,7 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
   __syncthreads();
   const int mij = (nx - 2) * (ny - 2);
   const unsigned x_bytes =
-      (unsigned)sizeof(T) * mij * ((k > 2) + (k < nz - 1));
+      (unsigned)sizeof(T) * mij * ((k > 2) + (k < nz - 1)) + a.extra_tx;
   constexpr unsigned kXcBytes =
       (unsigned)(offsetof(BcSmem<T>, omega) - offsetof(BcSmem<T>, xc) + 8 +
                  15) &
@@ -556,12 +557,13 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
   }
   if (tid == 0) {
     mbar_init(&sm.bar_c, 1);
-    mbar_expect_tx(&sm.bar_c, kXcBytes);
+    mbar_expect_tx(&sm.bar_c, kXcBytes + a.extra_tx);
     if (rank == 0) {
       mbar_init(&sm.bar_r, 1);
-      mbar_expect_tx(&sm.bar_r, (unsigned)sizeof(T) * mij * (nz - 2));
+      mbar_expect_tx(&sm.bar_r,
+                     (unsigned)sizeof(T) * mij * (nz - 2) + a.extra_tx);
       mbar_init(&sm.bar_d, 1);
-      mbar_expect_tx(&sm.bar_d, 16u * (nz - 2));
+      mbar_expect_tx(&sm.bar_d, 16u * (nz - 2) + a.extra_tx);
     }
   }
   fence_mbar_init();
@@ -633,7 +635,7 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
       // (every CTA takes delivery, also one without a plane: nothing is in
       // flight to it when it leaves)
       if (phase == 1 && rank != 0)
-        lost |= !mbar_wait_cluster(&sm.bar_c, 0);
+        lost |= !mbar_wait_cluster(&sm.bar_c, 0, lost);
       if (active) {
         if (phase == 1) {
           const int cy = cd.sy(), cz = cd.sz();
@@ -658,9 +660,9 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
             for (int q16 = 0; q16 < a.idle_delay; ++q16)
               __nanosleep(16384);
           if (s == 2 ? g == 0 : g == 1 || s > 0 || phase == 1) {
-            lost |= !mbar_wait_cluster(&sm.bar_x[g], x_parity);
+            lost |= !mbar_wait_cluster(&sm.bar_x[g], x_parity, lost);
             x_parity ^= 1u;
-            mbar_expect_tx_if(first, &sm.bar_x[g], x_bytes);
+            mbar_expect_tx_if(first && !lost, &sm.bar_x[g], x_bytes);
           }
           if (s == 2) {
             if (g == 0)
@@ -712,7 +714,7 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
       // ---- the levels below on rank 0, one point per thread in the order
       // of the colours ----
       if (rank == 0 && top == 2) {
-        lost |= !mbar_wait_cluster(&sm.bar_r, 0);
+        lost |= !mbar_wait_cluster(&sm.bar_r, 0, lost);
         if (t1 >= 0)
           level1();
       }
@@ -761,7 +763,7 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
             for (int t = 0; t < 27; ++t)
               w27[t] = mine ? b.P.p[t][pc] : T(0);
             if (st == 0) {
-              lost |= !mbar_wait_cluster(&sm.bar_r, 0);
+              lost |= !mbar_wait_cluster(&sm.bar_r, 0, lost);
               fl = bc_restrict_with<kBcRow, kBcPlane, kBcOdd>(sm.r, w27, li,
                                                               lj, lk);
             } else {
@@ -860,7 +862,7 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
   }
   if (rank == 0 && warp == 15) {
     // the damping of the top level, planes in order
-    lost |= !mbar_wait_cluster(&sm.bar_d, 0);
+    lost |= !mbar_wait_cluster(&sm.bar_d, 0, lost);
     double t0 = 0.0, t1 = 0.0;
     for (int p = 0; p < nz - 2; ++p) {
       t0 += sm.dsum[p][0];
@@ -870,8 +872,7 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
   }
   if (lost)
     *a.kernel_err = 1;
-  settle_if(lost);
-  cluster.sync(); // no CTA leaves while another may still send to it
+  leave_cluster(lost);
 }
 
 __global__ void __cluster_dims__(kCgCtas, 1, 1)

@@ -60,6 +60,11 @@ struct CgArgs {
   double *omega;
   int max_iters;
   int *status; // [0] iterations, the class: [1] stopped by the cap
+  // set to err_value, after status, when a message did not arrive (a bounded
+  // wait ran out)
+  int *err;
+  int err_value;
+  unsigned extra_tx; // a test's bytes that no message brings (0)
 };
 
 inline bool cg_cluster_fits(const Dims &d) {
@@ -150,7 +155,8 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
   // Messages (C > 1). The r.r sum also waits for the neighbours' r on the
   // copied planes, so its bytes include them; the senders store each r with
   // its bytes on the neighbour's mbarrier.
-  unsigned msg_bytes[2] = {8u * C, 8u * C}, parity[2] = {0u, 0u};
+  unsigned msg_bytes[2] = {8u * C + a.extra_tx, 8u * C + a.extra_tx};
+  unsigned parity[2] = {0u, 0u};
   unsigned dn = 0, dn_bar = 0, up = 0, up_bar = 0; // cluster addresses
   bool lost = false;
   if constexpr (C > 1) {
@@ -221,9 +227,9 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     if constexpr (C > 1) {
       send(cluster_addr(&sCta[set][rank], lane & (C - 1)), v,
            tid < C ? cluster_addr(&bar[set], lane & (C - 1)) : 0u);
-      lost |= !mbar_wait_cluster(&bar[set], parity[set]);
+      lost |= !mbar_wait_cluster(&bar[set], parity[set], lost);
       parity[set] ^= 1u;
-      mbar_expect_tx_if(tid == 0, &bar[set], msg_bytes[set]);
+      mbar_expect_tx_if(tid == 0 && !lost, &bar[set], msg_bytes[set]);
       const double *t = sCta[set];
       v = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
       static_assert(C == 8, "the tree of the CTAs' sums");
@@ -260,10 +266,13 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     }
     // (threads that gave a message up may hold other sums than the rest of
     // the CTA: every branch on a sum comes after a vote on that)
-    if constexpr (C == 1)
+    if constexpr (C == 1) {
       __syncthreads();
-    else if (__syncthreads_or(lost))
-      break;
+    } else {
+      lost = __syncthreads_or(lost);
+      if (lost)
+        break;
+    }
     if constexpr (APBS) {
       if ((it == 0 && (r0 == 0.0 || r0 / r0 <= a.errtol)) ||
           (it > 0 && rs <= stop2) || it >= a.max_iters)
@@ -281,8 +290,11 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     apv = row.apply(pval);
     const double pap = allsum(apv * pv, 1);
     if (!APBS && it == 0) {
-      if (C > 1 && __syncthreads_or(lost))
-        break;
+      if constexpr (C > 1) {
+        lost = __syncthreads_or(lost);
+        if (lost)
+          break;
+      }
       if (pap == 0.0)
         break;
       const double res = a.class_first_check ? sqrt(r0) : r0;
@@ -300,7 +312,7 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     rs = allsum(rv * rv, 0);
   }
   if constexpr (!APBS)
-    if (a.omega) {
+    if (a.omega && !lost) {
       // the damping (f . x) / (x . A x), x exchanged like r. (The sums'
       // sets alternate: the last one was r.r unless no iteration ran.)
       if (it > 0)
@@ -335,14 +347,14 @@ __device__ __forceinline__ void cg_on_chip(const CgArgs &a) {
     }
   }
   if (rank == 0 && tid == 0) {
-    // a lost message (never seen) is reported like the cap
-    a.status[0] = APBS && lost ? -1 : it;
+    a.status[0] = it;
     if constexpr (!APBS)
-      a.status[1] = capped || lost ? 1 : 0;
+      a.status[1] = capped ? 1 : 0;
   }
   if constexpr (C > 1) {
-    settle_if(lost);
-    cgs::this_cluster().sync(); // no CTA leaves while another sends to it
+    leave_cluster(lost);
+    if (lost && a.err)
+      *a.err = a.err_value;
   }
 }
 
@@ -359,7 +371,8 @@ __global__ void __launch_bounds__(kCgCtaThreads)
 
 // One solve of a level that cg_cluster_fits, queued on s.
 template <int KIND, bool APBS>
-int launch_cg_on_chip(const CgArgs &a, cudaStream_t s) {
+int launch_cg_on_chip(CgArgs a, cudaStream_t s) {
+  a.extra_tx = test_message_extra_tx();
   const int mk = a.d.nz - 2;
   if (cg_one_cta(a.d))
     cg_cta_kernel<KIND, APBS><<<1, cg_threads(a.d, mk), 0, s>>>(a);

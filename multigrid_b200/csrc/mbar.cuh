@@ -124,10 +124,19 @@ __device__ __forceinline__ void copy_to_cta_if(bool on, unsigned dst,
                "r"(smem_addr(src)), "r"(bytes), "r"(bar), "r"((unsigned)on)
                : "memory");
 }
-// mbar_wait for messages: what the senders wrote before them is visible
+// Polls for a message before it counts as lost: the hardware suspends a poll
+// that finds nothing for about 4 us, so a quarter of a second, ten times the
+// longest wait there is (a CTA waiting out 20000 iterations of the level-1 CG
+// in another).
+constexpr int kMessagePolls = 1 << 16;
+
+// mbar_wait for messages: what the senders wrote before them is visible. A
+// thread that has lost a message before looks once and goes on.
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar,
-                                                  unsigned parity) {
-  for (long polls = 0; polls < kTmaMaxPolls; ++polls) {
+                                                  unsigned parity,
+                                                  bool lost) {
+  const int limit = lost ? 1 : kMessagePolls;
+  for (int polls = 0; polls < limit; ++polls) {
     unsigned done;
     asm volatile("{\n"
                  ".reg .pred p;\n"
@@ -144,10 +153,15 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar,
   return false;
 }
 
-// After a lost message: time for this thread's own messages and copies in
-// flight to land before its CTA lets the cluster's last barrier pass (about
-// 1 ms, some 10^3 times a message).
-__device__ __forceinline__ void settle_if(bool lost) {
+// The end of a kernel whose CTAs send to each other: no CTA leaves while
+// another may still send to it. A CTA that has received everything it expects
+// can leave after the barrier; one with a thread that lost a message stays
+// another millisecond (some 10^3 times a message), so that what was sent to
+// it before the barrier lands in its own memory.
+__device__ __forceinline__ void leave_cluster(bool lost) {
+  asm volatile("barrier.cluster.arrive;\n"
+               "barrier.cluster.wait;\n" ::
+                   : "memory");
   if (lost)
     for (int q = 0; q < 64; ++q)
       __nanosleep(16384);

@@ -149,8 +149,8 @@ struct CghsScratch {
 template <int KIND>
 int cghs_on_chip(const Dims &d, const Op14<double> &A, const double *cc,
                  const double *fc, double *x, double *pv, double *ap,
-                 double *r, int itmax, int *it, double errtol,
-                 cudaStream_t s) {
+                 double *r, int itmax, int *it, int *err, int err_value,
+                 double errtol, cudaStream_t s) {
   // p's shell reads as zero afterwards, as the general path leaves it
   PMG_CUDA_TRY(cudaMemsetAsync(pv, 0, sizeof(double) * d.count(), s));
   CgArgs a{};
@@ -165,6 +165,8 @@ int cghs_on_chip(const Dims &d, const Op14<double> &A, const double *cc,
   a.errtol = errtol;
   a.max_iters = itmax;
   a.status = it;
+  a.err = err;
+  a.err_value = err_value;
   return launch_cg_on_chip<KIND, true>(a, s);
 }
 
@@ -178,7 +180,7 @@ int cghs(const Dims &d, const Op14<double> &A, const double *cc,
   if (cg_cluster_fits(d)) {
     int *it = nullptr;
     PMG_CUDA_TRY(scratch_alloc((void **)&it, sizeof(int), s));
-    int rc = cghs_on_chip<KIND>(d, A, cc, fc, x, pv, ap, r, itmax, it,
+    int rc = cghs_on_chip<KIND>(d, A, cc, fc, x, pv, ap, r, itmax, it, it, -1,
                                 errtol, s);
     cudaError_t e = cudaSuccess;
     if (rc == PMG_OK)
@@ -193,7 +195,8 @@ int cghs(const Dims &d, const Op14<double> &A, const double *cc,
       return PMG_ERR_CUDA;
     }
     if (*iters < 0) {
-      set_last_message("Vcghs: a message between CTAs did not arrive");
+      set_last_message("Vcghs: a message between CTAs did not arrive "
+                       "(bounded wait ran out)");
       *iters = 0;
       return PMG_ERR_TIMEOUT;
     }
@@ -843,9 +846,10 @@ struct ApbsDriver {
                 double *ap, double *r, int itmax, double errtol) {
     int *it = (int *)(ticket + 1);
     return L.kind == 7 ? cghs_on_chip<7>(L.d, level_op(L), L.cc, f, x, p, ap,
-                                         r, itmax, it, errtol, s)
+                                         r, itmax, it, nullptr, 0, errtol, s)
                        : cghs_on_chip<27>(L.d, level_op(L), L.cc, f, x, p,
-                                          ap, r, itmax, it, errtol, s);
+                                          ap, r, itmax, it, nullptr, 0,
+                                          errtol, s);
   }
 
   // Vsmooth (smoothd.cc:58-87): red-black GS (then the residual into w1

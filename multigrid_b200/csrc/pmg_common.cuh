@@ -217,6 +217,9 @@ template <auto Kernel> cudaError_t set_smem_limit(int bytes) {
   } while (0)
 
 namespace pmg {
+// pmg_test_message_short_delivery: extra bytes every wait for messages
+// between CTAs expects
+unsigned test_message_extra_tx();
 void set_last_error(cudaError_t e, const char *what, const char *file,
                     int line);
 void set_last_message(const char *msg);

@@ -311,6 +311,9 @@ __global__ void __launch_bounds__(1024)
   }
 }
 
+static std::atomic<unsigned> g_message_extra_tx{0};
+unsigned test_message_extra_tx() { return g_message_extra_tx.load(); }
+
 int launch_cg_level(const Dims &d, const Op14<double> &A, const double *rhs,
                     double *x, double *r, double *p, double *ap,
                     double thresh, double rel_tol, int class_first_check,
@@ -327,6 +330,8 @@ int launch_cg_level(const Dims &d, const Op14<double> &A, const double *rhs,
     a.class_first_check = class_first_check;
     a.max_iters = max_iters;
     a.status = status;
+    a.err = status + 1;
+    a.err_value = 2;
     return launch_cg_on_chip<27, false>(a, s);
   }
   const long m = (long)(d.nx - 2) * (d.ny - 2) * (d.nz - 2);
@@ -950,10 +955,22 @@ int pmg_cg_level_d(int nx, int ny, int nz, const double *const *a14,
   if (iters)
     *iters = host_status[0];
   if (host_status[1]) {
-    set_last_message("cg_level: iteration cap reached above the threshold");
+    set_last_message(host_status[1] == 2
+                         ? "cg_level: a message between CTAs did not arrive "
+                           "(bounded wait ran out)"
+                         : "cg_level: iteration cap reached above the "
+                           "threshold");
     rc = PMG_ERR_TIMEOUT;
   }
   return rc;
+}
+
+int pmg_test_message_short_delivery(int bytes) {
+  PMG_REQUIRE(bytes >= 0 && bytes % 16 == 0 && bytes <= (1 << 16),
+              "pmg_test_message_short_delivery: bytes must be a multiple of "
+              "16 in [0, 2^16]");
+  g_message_extra_tx.store((unsigned)bytes);
+  return PMG_OK;
 }
 
 } // extern "C"

@@ -95,8 +95,11 @@ extern "C" int pmg_cg_level_noalloc_d(int nx, int ny, int nz,
   if (iters)
     *iters = host_status[0];
   if (host_status[1]) {
-    set_last_message(
-        "cg_level_noalloc: iteration cap reached above the threshold");
+    set_last_message(host_status[1] == 2
+                         ? "cg_level_noalloc: a message between CTAs did not "
+                           "arrive (bounded wait ran out)"
+                         : "cg_level_noalloc: iteration cap reached above "
+                           "the threshold");
     return PMG_ERR_TIMEOUT;
   }
   return PMG_OK;

@@ -195,7 +195,8 @@ struct pmg_problem {
   double *inv1 = nullptr;
   int *inv1_ok = nullptr;
   // device: set by the staged kernels (gs27_tma_kernel, gs7_stream_kernel,
-  // defect_norm_stream_kernel) on a lost stage
+  // defect_norm_stream_kernel) on a lost stage and by the kernels of the
+  // lowest levels (bottom_cluster.cuh, cg_cluster.cuh) on a lost message
   int *kernel_err = nullptr;
   int num_sms = 0;
   // Relative stopping threshold of the coarsest CG on the mixed path's
@@ -263,6 +264,11 @@ std::atomic<int> g_stream_on{1};
 std::atomic<unsigned> g_tma_extra_tx{0};
 // pmg_test_idle_warp_delay, in units of 16 us
 std::atomic<int> g_idle_delay{0};
+
+const char kLostMessage[] =
+    "pmg_solve: a staged copy (27-point smoother, streamed finest pass or "
+    "residual) or a message between CTAs (lowest levels) did not arrive "
+    "(bounded wait ran out)";
 
 int level_n(int base, int L) { return base * (1 << L) + 1; }
 
@@ -517,6 +523,8 @@ int cg_level1(pmg_problem *p) {
     a.class_first_check = fp64;
     a.max_iters = kCgMaxIters;
     a.status = p->cg_status;
+    a.err = p->kernel_err;
+    a.err_value = 1;
     return launch_cg_on_chip<27, false>(a, s);
   }
   if (mixed)
@@ -567,6 +575,7 @@ template <typename T> BottomArgs<T> bottom_args(pmg_problem *p, int top) {
   a.inv = p->inv1;
   a.inv_ok = p->inv1_ok;
   a.idle_delay = g_idle_delay.load();
+  a.extra_tx = test_message_extra_tx();
   return a;
 }
 
@@ -2070,9 +2079,7 @@ static int solve_host_loop(pmg_problem *p, double tol, int max_cycles,
   PMG_CUDA_TRY(cudaMemcpy(&lost, p->kernel_err, sizeof(int),
                           cudaMemcpyDeviceToHost));
   if (rc == PMG_OK && lost) {
-    set_last_message("pmg_solve: a staged copy (27-point smoother, "
-                     "streamed finest pass or residual) did not arrive "
-                     "(bounded wait ran out)");
+    set_last_message(kLostMessage);
     rc = PMG_ERR_TIMEOUT;
   }
   return rc;
@@ -2154,9 +2161,7 @@ int pmg_solve_finish(pmg_problem *p, int *cycles, double *relres,
     return PMG_ERR_DIVERGED;
   }
   if (st.status == 3) {
-    set_last_message("pmg_solve: a staged copy (27-point smoother, "
-                     "streamed finest pass or residual) did not arrive "
-                     "(bounded wait ran out)");
+    set_last_message(kLostMessage);
     return PMG_ERR_TIMEOUT;
   }
   return PMG_OK;

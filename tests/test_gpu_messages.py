@@ -1,5 +1,8 @@
 """Messages between the CTAs of the kernels that hold the lowest levels on
-chip: their order against late warps."""
+chip: their order against late warps, and what a caller sees when one does
+not arrive (every wait expects 16 bytes more than are sent and runs out)."""
+import contextlib
+
 import numpy as np
 import pytest
 
@@ -10,7 +13,8 @@ pytestmark = pytest.mark.gpu
 if not torch.cuda.is_available():  # pragma: no cover
     pytest.skip("no CUDA device", allow_module_level=True)
 
-from multigrid_b200 import PBELinearProblem, _lib  # noqa: E402
+from multigrid_b200 import PBELinearProblem, _lib, pmgc  # noqa: E402
+from multigrid_b200._lib import PmgError  # noqa: E402
 from multigrid_b200.molecule import Workload, level_n  # noqa: E402
 from multigrid_b200.problem import setup_fine  # noqa: E402
 
@@ -47,3 +51,67 @@ def test_late_warps_without_a_point(base, nlev, precision):
                    _lib.lib.pmg_test_idle_warp_delay(0))
     assert got[0] == want[0]
     assert np.array_equal(got[1], want[1])
+
+
+@contextlib.contextmanager
+def messages_lost():
+    _lib.check("pmg_test_message_short_delivery",
+               _lib.lib.pmg_test_message_short_delivery(16))
+    try:
+        yield
+    finally:
+        _lib.check("pmg_test_message_short_delivery",
+                   _lib.lib.pmg_test_message_short_delivery(0))
+
+
+def reports_lost(call):
+    with pytest.raises(PmgError) as e:
+        call()
+    assert e.value.status == _lib.PMG_ERR_TIMEOUT
+    assert b"did not arrive" in _lib.lib.pmg_last_error()
+
+
+def dominant(n, seed):
+    rng = np.random.default_rng(seed)
+    ops = [np.full(n ** 3, 27.0)] + [rng.uniform(0.0, 1.0, n ** 3)
+                                     for _ in range(13)]
+    return (torch.as_tensor(np.stack(ops), device="cuda"),
+            torch.as_tensor(rng.normal(size=n ** 3), device="cuda"))
+
+
+# one and two planes per CTA
+@pytest.mark.parametrize("n", [10, 17])
+def test_lost_message_of_the_cg_is_reported(n):
+    ops, f = dominant(n, n)
+
+    def cg():
+        x = torch.zeros_like(f)
+        it = pmgc.cg_level(n, n, n, list(ops), f, x)
+        return it, x
+
+    def vcghs():
+        x = torch.zeros_like(f)
+        work = [torch.zeros_like(f) for _ in range(3)]
+        it = pmgc.Vcghs(n, n, n, ops, torch.zeros_like(f), f, x, *work, 200,
+                        1e-10)
+        return it, x
+
+    for call in (cg, vcghs):
+        want = call()
+        with messages_lost():
+            reports_lost(call)
+        got = call()
+        assert got[0] == want[0] and torch.equal(got[1], want[1])
+
+
+# levels 5^3 to 17^3, 5^3 and 9^3 and 7^3 and 13^3 in one launch; a level 1 of
+# 11^3 by itself
+@pytest.mark.parametrize("precision", ["mixed", "fp64", "fp64-fast"])
+@pytest.mark.parametrize("base,nlev", [(2, 4), (2, 3), (3, 3), (5, 2)])
+def test_lost_message_of_a_solve_is_reported(base, nlev, precision):
+    w, fine = problem(base, nlev)
+    want = solve(w, fine, precision)
+    with messages_lost():
+        reports_lost(lambda: solve(w, fine, precision))
+    got = solve(w, fine, precision)
+    assert got[0] == want[0] and np.array_equal(got[1], want[1])
