@@ -8,6 +8,7 @@
 // uC oNE oNW uE uW uN uS uNE uNW uSE uSW (27-point, 14 columns); ipc[10]
 // (the reference's VAT(ipc, 11)) is 7 or 27.
 #include <algorithm>
+#include <string.h>
 #include <type_traits>
 
 #include "cg_cluster.cuh"
@@ -798,6 +799,8 @@ struct ApbsDriver {
   ApbsLevel lv[13];
   double *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
   void *block = nullptr; // every level array and work vector
+  // res: the reductions' results (two), a lost-message word (int, set by the
+  // queued Vcghs solves), the damping
   double *partials = nullptr, *res = nullptr;
   unsigned *ticket = nullptr;
 
@@ -811,10 +814,21 @@ struct ApbsDriver {
     return ReduceSlot{partials, ticket, out};
   }
 
-  int fetch(const double *dev, double *host) {
-    PMG_CUDA_TRY(cudaMemcpyAsync(host, dev, sizeof(double),
-                                 cudaMemcpyDeviceToHost, s));
+  // the last reduction's result, and whether a queued solve before it lost a
+  // message
+  int fetch(double *host) {
+    double v[3];
+    PMG_CUDA_TRY(cudaMemcpyAsync(v, res, sizeof(v), cudaMemcpyDeviceToHost,
+                                 s));
     PMG_CUDA_TRY(cudaStreamSynchronize(s));
+    int lost;
+    memcpy(&lost, &v[2], sizeof(lost));
+    if (lost) {
+      set_last_message("Vmvcs: a message between CTAs of the CG did not "
+                       "arrive (bounded wait ran out)");
+      return PMG_ERR_TIMEOUT;
+    }
+    *host = v[0];
     return PMG_OK;
   }
 
@@ -837,19 +851,19 @@ struct ApbsDriver {
     apbs_sum_kernel<<<reduce_grid(L.d), interior_block(), 0, s>>>(
         L.d, a, b, mode, slot(res));
     PMG_LAUNCH_CHECK();
-    return fetch(res, host);
+    return fetch(host);
   }
 
   // Vcghs of a level that fits on chip, queued: nothing in the cycle reads
-  // its iteration count
+  // its iteration count; a lost message comes back with the stop test's norm
   int cg_queued(ApbsLevel &L, const double *f, double *x, double *p,
                 double *ap, double *r, int itmax, double errtol) {
-    int *it = (int *)(ticket + 1);
+    int *it = (int *)(ticket + 1), *err = (int *)(res + 2);
     return L.kind == 7 ? cghs_on_chip<7>(L.d, level_op(L), L.cc, f, x, p, ap,
-                                         r, itmax, it, nullptr, 0, errtol, s)
+                                         r, itmax, it, err, 1, errtol, s)
                        : cghs_on_chip<27>(L.d, level_op(L), L.cc, f, x, p,
-                                          ap, r, itmax, it, nullptr, 0,
-                                          errtol, s);
+                                          ap, r, itmax, it, err, 1, errtol,
+                                          s);
   }
 
   // Vsmooth (smoothd.cc:58-87): red-black GS (then the residual into w1
@@ -916,7 +930,7 @@ struct ApbsDriver {
                 F.d, level_op(F), F.cc, F.fc, F.x, w1, slot(res));
       });
       PMG_LAUNCH_CHECK();
-      return fetch(res, out);
+      return fetch(out);
     }
     const int rc = sum(F, tru, F.x, istop == 2 ? 2 : 3, out);
     if (rc == PMG_OK && istop == 3)

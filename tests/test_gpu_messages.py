@@ -17,6 +17,7 @@ from multigrid_b200 import PBELinearProblem, _lib, pmgc  # noqa: E402
 from multigrid_b200._lib import PmgError  # noqa: E402
 from multigrid_b200.molecule import Workload, level_n  # noqa: E402
 from multigrid_b200.problem import setup_fine  # noqa: E402
+from test_oracle import apbs_maps, apbs_params  # noqa: E402
 
 
 def problem(base, nlev):
@@ -115,3 +116,28 @@ def test_lost_message_of_a_solve_is_reported(base, nlev, precision):
         reports_lost(lambda: solve(w, fine, precision))
     got = solve(w, fine, precision)
     assert got[0] == want[0] and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("kw", [dict(nlev=2), dict(nlev=1),
+                                dict(nlev=2, mgsmoo=4, itmax=3)])
+def test_lost_message_of_the_driver_is_reported(kw):
+    """The driver queues its coarsest CG (17^3 here) and, with mgsmoo 4, the
+    smoother's without reading them back; the stop test's norm brings the
+    loss."""
+    n = 33 if kw["nlev"] == 2 else 17
+    maps = apbs_maps(n, n)
+    iparm, rparm = apbs_params(n, **kw)
+    dev = [torch.as_tensor(np.ascontiguousarray(maps[k]), device="cuda",
+                           dtype=torch.float64)
+           for k in ("xf", "yf", "zf", "gxcf", "gycf", "gzcf", "a1cf", "a2cf",
+                     "a3cf", "ccf", "fcf")]
+
+    def drive():
+        u = torch.zeros(n ** 3, dtype=torch.float64, device="cuda")
+        return pmgc.Vmgdriv(iparm, rparm, u, *dev), u
+
+    want = drive()
+    with messages_lost():
+        reports_lost(drive)
+    got = drive()
+    assert got[0] == want[0] and torch.equal(got[1], want[1])
