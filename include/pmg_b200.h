@@ -627,8 +627,9 @@ int pmg_solve(pmg_problem *p, double tol, int max_cycles, int *cycles,
  * times its initial value (tol = 0: the app's counting criterion). The
  * result replaces the finest iterate (pmg_get_potential); *iters, *relres
  * and hist (max_iters + 1 entries, may be NULL) as for pmg_solve. The whole
- * iteration is one graph launch (stop test on the GPU). Allocates 6 n^3
- * doubles on first use. */
+ * iteration is one graph launch (stop test on the GPU); a bounded wait that
+ * runs out in it is reported as pmg_solve reports it. Allocates 6 n^3 doubles
+ * on first use. */
 int pmg_pcg_solve(pmg_problem *p, double tol, int max_iters, int *iters,
                   double *relres, double *hist);
 

@@ -17,7 +17,9 @@ struct PcgState {
   double tol;
   int max_iters;
   int iters;
-  int status; // 0 ok / stopped, 1 diverged, 2 initial residual not finite
+  // 0 ok / stopped, 1 diverged, 2 initial residual not finite, 3 a staged
+  // copy or a message did not arrive
+  int status;
   int pad;
   double rs, alpha, beta, r0, rn;
   double hist[1025];
@@ -117,15 +119,18 @@ __global__ void pcg_params_kernel(PcgState *st, double tol, int max_iters) {
 // 110-116) or the initial residual is zero or not finite
 __global__ void pcg_init_kernel(PcgState *st, const double *rr,
                                 const double *rz, const double *pap,
-                                double n3, cudaGraphConditionalHandle h) {
+                                double n3, const int *kernel_err,
+                                cudaGraphConditionalHandle h) {
   const double r0 = sqrt(rr[0] / n3);
   st->r0 = r0;
   st->rn = r0;
   st->hist[0] = r0;
   st->rs = rz[0];
   const bool finite = isfinite(r0);
-  st->status = finite ? 0 : 2;
-  const bool go = finite && r0 > 0.0 && pap[0] != 0.0 && st->max_iters > 0;
+  const bool lost = *kernel_err != 0;
+  st->status = lost ? 3 : finite ? 0 : 2;
+  const bool go = !lost && finite && r0 > 0.0 && pap[0] != 0.0 &&
+                  st->max_iters > 0;
   st->alpha = pap[0] != 0.0 ? st->rs / pap[0] : 0.0;
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
@@ -140,6 +145,7 @@ __global__ void pcg_beta_kernel(PcgState *st, const double *rz) {
 // residual's norm sqrt(sum r^2 / n^3) relative to the initial one
 __global__ void pcg_check_kernel(PcgState *st, const double *pap,
                                  const double *rr, double n3,
+                                 const int *kernel_err,
                                  cudaGraphConditionalHandle h) {
   st->alpha = pap[0] == 0.0 ? 0.0 : st->rs / pap[0];
   const int c = ++st->iters;
@@ -148,11 +154,14 @@ __global__ void pcg_check_kernel(PcgState *st, const double *pap,
   if (c <= 1024)
     st->hist[c] = rn;
   const bool diverged = !isfinite(rn) || rn > 1e6 * st->r0;
+  const bool lost = *kernel_err != 0;
   if (diverged)
     st->status = 1;
+  if (lost)
+    st->status = 3;
   const bool converged = st->tol > 0.0 && rn / st->r0 < st->tol;
   cudaGraphSetConditional(
-      h, (!diverged && !converged && c < st->max_iters) ? 1u : 0u);
+      h, (!diverged && !lost && !converged && c < st->max_iters) ? 1u : 0u);
 }
 
 } // namespace pmg

@@ -266,7 +266,7 @@ std::atomic<unsigned> g_tma_extra_tx{0};
 std::atomic<int> g_idle_delay{0};
 
 const char kLostMessage[] =
-    "pmg_solve: a staged copy (27-point smoother, streamed finest pass or "
+    "a staged copy (27-point smoother, streamed finest pass or "
     "residual) or a message between CTAs (lowest levels) did not arrive "
     "(bounded wait ran out)";
 
@@ -1471,7 +1471,7 @@ int ensure_pcg_graph(pmg_problem *p) {
     pcg_dot_kernel<<<rg, rb, 0, s>>>(v.d, c.r, c.z, c.rz);
     matvec();
     pcg_init_kernel<<<1, 1, 0, s>>>(c.d_st, c.rr.result, c.rz.result,
-                                    c.pap.result, n3, h);
+                                    c.pap.result, n3, p->kernel_err, h);
     PMG_LAUNCH_CHECK();
     return PMG_OK;
   };
@@ -1509,7 +1509,7 @@ int ensure_pcg_graph(pmg_problem *p) {
     pcg_update_p_kernel<<<rg, rb, 0, s>>>(v.d, c.z, c.pv, c.d_st);
     matvec();
     pcg_check_kernel<<<1, 1, 0, s>>>(c.d_st, c.pap.result, c.rr.result, n3,
-                                     h);
+                                     p->kernel_err, h);
     PMG_LAUNCH_CHECK();
     return PMG_OK;
   };
@@ -2208,6 +2208,7 @@ int pmg_pcg_solve(pmg_problem *p, double tol, int max_iters, int *iters,
     rc = ensure_pcg_graph(p);
   if (rc)
     return rc;
+  PMG_CUDA_TRY(cudaMemsetAsync(p->kernel_err, 0, sizeof(int), p->stream));
   pcg_params_kernel<<<1, 1, 0, p->stream>>>(p->pcg.d_st, tol, max_iters);
   PMG_LAUNCH_CHECK();
   PMG_CUDA_TRY(cudaGraphLaunch(p->pcg.exec, p->stream));
@@ -2229,6 +2230,10 @@ int pmg_pcg_solve(pmg_problem *p, double tol, int max_iters, int *iters,
   if (st.status == 1) {
     set_last_message("pmg_pcg_solve: residual diverged");
     return PMG_ERR_DIVERGED;
+  }
+  if (st.status == 3) {
+    set_last_message(kLostMessage);
+    return PMG_ERR_TIMEOUT;
   }
   return PMG_OK;
 }

@@ -141,3 +141,23 @@ def test_lost_message_of_the_driver_is_reported(kw):
         reports_lost(drive)
     got = drive()
     assert got[0] == want[0] and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64", "fp64-fast"])
+@pytest.mark.parametrize("base,nlev", [(2, 4), (5, 2)])
+def test_lost_message_of_a_pcg_solve_is_reported(base, nlev, precision):
+    w, fine = problem(base, nlev)
+
+    def pcg():
+        with PBELinearProblem(w.base, w.nlev, w.box, precision,
+                              w.physics) as p:
+            p.set_fine(**fine)
+            p.buildmultilevelops()
+            r = p.pcg_solve(tol=1e-10, max_iters=60)
+            return r.cycles, p.potential().ravel().copy()
+
+    want = pcg()
+    with messages_lost():
+        reports_lost(pcg)
+    got = pcg()
+    assert got[0] == want[0] and np.array_equal(got[1], want[1])
