@@ -598,7 +598,9 @@ int pmg_build_hierarchy(pmg_problem *p, int trilinear);
 
 /* One V-cycle of the class (v_cycle, PBE_pmgc_class.h:1070-1114); with
  * as_preconditioner != 0 every level is zero-initialised. FP64 problems
- * only. */
+ * only. Queued on the problem's stream; a bounded wait that runs out in it is
+ * reported (PMG_ERR_TIMEOUT, once) by the next pmg_compute_residual_2 or
+ * pmg_get_potential. */
 int pmg_vcycle(pmg_problem *p, int as_preconditioner);
 
 /* sqrt(sum_interior (f - A x)^2 / n^3) of the finest level; synchronises.

@@ -209,7 +209,7 @@ struct pmg_problem {
   // both passes of plan() lay out the same arrays)
   bool tma_on = true;
   ReduceSlot red_norm{}, red_lambda{};
-  double *h_pinned = nullptr; // [0] residual sum, [1..] spare
+  double *h_pinned = nullptr; // [0] residual sum, [1] kernel_err, spare
   int *h_status = nullptr;
   bool fine_set = false, built = false;
   // One V-cycle (plus the residual norm) captured as a CUDA graph.
@@ -222,6 +222,9 @@ struct pmg_problem {
   SolveState *h_state = nullptr; // pinned
   cudaEvent_t done_ev = nullptr;
   bool solve_pending = false;
+  // pmg_vcycle has queued (or captured) cycles of the caller's: the calls
+  // that wait for the stream look at kernel_err
+  bool caller_cycles = false;
   bool host_loop = false; // pmg_problem_set_host_loop
   bool use_codes = true;   // pmg_problem_set_coded_couplings
   // the finest colour passes stream their rows through shared memory
@@ -2010,7 +2013,30 @@ int pmg_vcycle(pmg_problem *p, int as_preconditioner) {
     set_last_message("pmg_vcycle: FP64 problems only");
     return PMG_ERR_ARG;
   }
+  p->caller_cycles = true;
   return vcycle64(p, p->nlev, as_preconditioner);
+}
+
+// A bounded wait ran out: told once, the word is clear for what comes next.
+static int report_lost(pmg_problem *p) {
+  PMG_CUDA_TRY(cudaMemsetAsync(p->kernel_err, 0, sizeof(int), p->stream));
+  set_last_message(kLostMessage);
+  return PMG_ERR_TIMEOUT;
+}
+
+// Around a call's wait for the stream, where the caller runs cycles of its
+// own: queues the read of the error word, and afterwards reports it.
+static int queue_lost_check(pmg_problem *p) {
+  if (p->caller_cycles)
+    PMG_CUDA_TRY(cudaMemcpyAsync(p->h_pinned + 1, p->kernel_err, sizeof(int),
+                                 cudaMemcpyDeviceToHost, p->stream));
+  return PMG_OK;
+}
+static int lost_in_cycles(pmg_problem *p) {
+  int lost = 0;
+  if (p->caller_cycles)
+    memcpy(&lost, p->h_pinned + 1, sizeof(lost));
+  return lost ? report_lost(p) : PMG_OK;
 }
 
 int pmg_compute_residual_2(pmg_problem *p, double *out) {
@@ -2019,11 +2045,13 @@ int pmg_compute_residual_2(pmg_problem *p, double *out) {
   if (!p->fine_set)
     return PMG_ERR_STATE;
   int rc = residual_norm_async(p);
+  if (!rc)
+    rc = queue_lost_check(p);
   if (rc)
     return rc;
   PMG_CUDA_TRY(cudaStreamSynchronize(p->stream));
   *out = norm_from_sum(p, p->h_pinned[0]);
-  return PMG_OK;
+  return lost_in_cycles(p);
 }
 
 // Host-driven loop: one cycle graph per launch and a residual read-back per
@@ -2078,10 +2106,8 @@ static int solve_host_loop(pmg_problem *p, double tol, int max_cycles,
   int lost = 0;
   PMG_CUDA_TRY(cudaMemcpy(&lost, p->kernel_err, sizeof(int),
                           cudaMemcpyDeviceToHost));
-  if (rc == PMG_OK && lost) {
-    set_last_message(kLostMessage);
-    rc = PMG_ERR_TIMEOUT;
-  }
+  if (rc == PMG_OK && lost)
+    rc = report_lost(p);
   return rc;
 }
 
@@ -2160,10 +2186,8 @@ int pmg_solve_finish(pmg_problem *p, int *cycles, double *relres,
     set_last_message("pmg_solve: residual diverged");
     return PMG_ERR_DIVERGED;
   }
-  if (st.status == 3) {
-    set_last_message(kLostMessage);
-    return PMG_ERR_TIMEOUT;
-  }
+  if (st.status == 3)
+    return report_lost(p);
   return PMG_OK;
 }
 
@@ -2231,10 +2255,8 @@ int pmg_pcg_solve(pmg_problem *p, double tol, int max_iters, int *iters,
     set_last_message("pmg_pcg_solve: residual diverged");
     return PMG_ERR_DIVERGED;
   }
-  if (st.status == 3) {
-    set_last_message(kLostMessage);
-    return PMG_ERR_TIMEOUT;
-  }
+  if (st.status == 3)
+    return report_lost(p);
   return PMG_OK;
 }
 
@@ -2244,8 +2266,11 @@ int pmg_get_potential(pmg_problem *p, double *dst) {
   LevelBuf &v = p->lv[p->nlev];
   PMG_CUDA_TRY(cudaMemcpyAsync(dst, v.x, sizeof(double) * v.n3,
                                cudaMemcpyDefault, p->stream));
+  const int rc = queue_lost_check(p);
+  if (rc)
+    return rc;
   PMG_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  return PMG_OK;
+  return lost_in_cycles(p);
 }
 
 int pmg_get_potential_async(pmg_problem *p, double *dst) {

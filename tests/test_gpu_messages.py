@@ -161,3 +161,49 @@ def test_lost_message_of_a_pcg_solve_is_reported(base, nlev, precision):
         reports_lost(pcg)
     got = pcg()
     assert got[0] == want[0] and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("base,nlev", [(2, 4), (5, 2)])
+def test_lost_message_of_a_caller_s_cycles_is_reported(base, nlev):
+    """Cycles queued one by one: the next call that waits for the stream
+    reports the loss, and only that one."""
+    w, fine = problem(base, nlev)
+
+    def run(end):
+        with PBELinearProblem(w.base, w.nlev, w.box, "fp64",
+                              w.physics) as p:
+            p.set_fine(**fine)
+            p.buildmultilevelops()
+            for _ in range(3):
+                p.v_cycle()
+            return end(p)
+
+    def residual(p):
+        return p.compute_residual_2()
+
+    def potential(p):
+        return p.potential().ravel().copy()
+
+    want = run(residual), run(potential)
+    for end in (residual, potential):
+        with messages_lost():
+            reports_lost(lambda: run(end))
+
+            def told_once(p):
+                reports_lost(lambda: end(p))
+                return end(p)
+
+            run(told_once)
+    assert run(residual) == want[0]
+    assert np.array_equal(run(potential), want[1])
+
+
+def test_cycles_after_a_solve_that_reported_a_loss():
+    w, fine = problem(2, 4)
+    with PBELinearProblem(w.base, w.nlev, w.box, "fp64", w.physics) as p:
+        p.set_fine(**fine)
+        p.buildmultilevelops()
+        with messages_lost():
+            reports_lost(lambda: p.solve(tol=1e-10, max_cycles=60))
+        p.v_cycle()
+        assert np.isfinite(p.compute_residual_2())
