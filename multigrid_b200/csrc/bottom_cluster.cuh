@@ -503,13 +503,15 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
   const BottomLevel<T> &v = a.lv[top];
   const Dims cd = a.lv[top - 1].d; // the level below the top
   StencilRow<T, 27> row;
-  T f = T(0), recip = T(0);
+  // (threads without a point: couplings of zero, and 1 / 1 in the divide, so
+  // that they stay on its short path)
+  T f = T(1), recip = T(1);
   auto load_row = [&]() {
     row.clear();
     if (own) {
       row.load(v.A, nullptr, gi, td.sy(), td.sz());
       f = v.f[gi];
-      recip = T(1) / row.centre;
+      recip = recip_of(row.centre);
     }
   };
   load_row();
@@ -725,9 +727,9 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
         const auto lp = split_point<kBlRow, kBlPlane, kBlOdd>(li, lj, lk - 1);
         StencilRow<T, 27> lrow;
         lrow.clear();
-        T lrecip = T(0);
+        T lrecip = T(1); // (1 / 1 again without a point)
         double omega = 0.0;
-        
+
         // down the levels and up again (one loop: their code once)
         const int down = top - 2;
 #pragma unroll 1
@@ -745,10 +747,10 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
           // (the first level up is the last one down: its row is here)
           auto load_local = [&]() {
             lrow.clear();
-            lrecip = T(0);
+            lrecip = T(1);
             if (mine) {
               lrow.load(b.A, nullptr, pc, b.d.sy(), b.d.sz());
-              lrecip = T(1) / lrow.centre;
+              lrecip = recip_of(lrow.centre);
             }
           };
           // (the row and the restriction's weights are loaded together where
@@ -756,7 +758,7 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
           constexpr bool kBoth = sizeof(T) == sizeof(float);
           if (st != down && (kBoth || ascend))
             load_local();
-          T fl = T(0);
+          T fl = T(1);
           if (!ascend) {
             T w27[27];
 #pragma unroll
@@ -773,6 +775,8 @@ __device__ __forceinline__ void bottom_cluster_body(const BottomArgs<T> &a) {
             }
             if (mine)
               lf[lp.c] = fl;
+            else
+              fl = T(1);
             if (!kBoth)
               load_local();
           } else {

@@ -26,18 +26,20 @@
 // double; the pass is bound more by instruction issue than by the copies). Plane k is computed
 // from the stages of k - 1, k and k + 1 while the next S - 3 planes are in
 // flight, so the bytes in flight are set by the ring, not by registers.
-// A warp computes a row, one point per lane. A point's seven coefficients and
-// the reciprocal of its divisor come from a 128-entry table in shared memory
+// A warp computes a row, one point per lane. A point's couplings and the
+// reciprocal of its divisor come from a 128-entry table in shared memory
 // indexed by its code byte (wide loads instead of six bit tests and selects
 // and a table lookup). The arithmetic is gs7_code_color_kernel's, term for
-// term, the divide as two corrections of the product with the reciprocal
-// (div_by_recip: the same bits), so the bits are the same. Before, a lane took
-// four consecutive points by 16-byte loads: rows of 33, 65 and 129 points
-// then need a round more than a multiple of 32 lanes (9, 17 and 33 quads),
-// and in double 96 registers left two CTAs per SM, with the IEEE divide in
-// every point. Per pass, float: 65^3 4.7 -> 3.75, 129^3 9.3 -> 7.4, 257^3 29.9 ->
-// 29.2 us (there 76 instructions per 32 points keep the issue slots 55% busy);
-// double: 129^3 21.9 -> 9.0, 161^3 32.8 -> 15.3 us.
+// term. The divide has its bits for every operand (row_stencil.cuh): in
+// double two corrections of the product with the reciprocal, in float one
+// double product with the reciprocal in two parts (the corrections need a
+// range test, whose branch cost more there: 257^3 mixed 21.8 -> 22.2 ms
+// against 21.9). Before, a lane took four consecutive points by 16-byte
+// loads: rows of 33, 65 and 129 points then need a round more than a multiple
+// of 32 lanes (9, 17 and 33 quads), and in double 96 registers left two CTAs
+// per SM, with the IEEE divide in every point. Per pass, float: 65^3 4.7 ->
+// 3.8, 129^3 9.1 -> 7.5, 257^3 29.8 -> 29.8 us (bound by instruction issue);
+// double: 129^3 21.8 -> 8.4, 161^3 32.4 -> 14.6 us.
 //
 // A pass reads only the other colour of x and writes only its own, so the
 // stages never hold values the pass changes. Rows and planes outside the
@@ -160,9 +162,27 @@ __device__ __forceinline__ void mbar_arrive_if(bool on, uint64_t *bar) {
                : "memory");
 }
 
-// half of a coefficient table row
-template <typename T> struct alignas(16) Quad {
-  T x, y, z, w;
+// Table row of a code byte: the six couplings in the order the update uses
+// them (n, s, e, w, down, up) and what the divide by oC + 0 needs
+// (row_stencil.cuh: the bits of the divide).
+template <typename T> struct StreamRow;
+template <> struct alignas(16) StreamRow<float> {
+  float c[8]; // (two spare)
+  RecipPair r;
+  __device__ __forceinline__ void set_centre(float oc) { r = recip_pair(oc); }
+  __device__ __forceinline__ float divide(float s) const {
+    return div_by_pair(s, r);
+  }
+};
+template <> struct alignas(16) StreamRow<double> {
+  double c[6], oc, y;
+  __device__ __forceinline__ void set_centre(double v) {
+    oc = v;
+    y = recip_of(v);
+  }
+  __device__ __forceinline__ double divide(double s) const {
+    return div_by_recip(s, oc, y);
+  }
 };
 
 // KEEP false: the first pass from a zero iterate (zero_initialize), whose
@@ -179,12 +199,9 @@ __global__ void __launch_bounds__(StreamCfg<T>::THREADS,
                       const T *__restrict__ octab,
                       const unsigned char *__restrict__ codeb, T *x,
                       int want, int *err, unsigned extra_tx) {
-  using V = Quad<T>;
   extern __shared__ __align__(128) unsigned char sm[];
-  // per code byte (its low seven bits) the point's seven coefficients in
-  // the order the update uses them: n, s, e, w, down, up, oC, and the
-  // reciprocal of oC (div_by_recip: the bits of the divide by oC + 0)
-  __shared__ __align__(16) T ctab[128][8];
+  // per code byte (its low seven bits)
+  __shared__ StreamRow<T> ctab[128];
   // full[s]: the slot's boxes landed (the producer's arrival and their
   // bytes); empty[s]: every consumer warp is done with it
   uint64_t *full = reinterpret_cast<uint64_t *>(sm + S * sh.slot);
@@ -211,15 +228,14 @@ __global__ void __launch_bounds__(StreamCfg<T>::THREADS,
   const bool oc_coded = coded && info[8] == 0;
   if (oc_coded && threadIdx.x < 128) {
     const unsigned b = threadIdx.x;
-    T *t = ctab[b];
-    t[0] = (b & 4u) ? L.nh : L.nl;
-    t[1] = (b & 8u) ? L.nh : L.nl;
-    t[2] = (b & 1u) ? L.eh : L.el;
-    t[3] = (b & 2u) ? L.eh : L.el;
-    t[4] = (b & 32u) ? L.uh : L.ul;
-    t[5] = (b & 16u) ? L.uh : L.ul;
-    t[6] = octab[b];
-    t[7] = T(1) / t[6];
+    StreamRow<T> &t = ctab[b];
+    t.c[0] = (b & 4u) ? L.nh : L.nl;
+    t.c[1] = (b & 8u) ? L.nh : L.nl;
+    t.c[2] = (b & 1u) ? L.eh : L.el;
+    t.c[3] = (b & 2u) ? L.eh : L.el;
+    t.c[4] = (b & 32u) ? L.uh : L.ul;
+    t.c[5] = (b & 16u) ? L.uh : L.ul;
+    t.set_centre(octab[b]);
   }
   __syncthreads();
   auto slot_of = [&](int kk) { return (kk - kfirst) % S; };
@@ -313,12 +329,10 @@ __global__ void __launch_bounds__(StreamCfg<T>::THREADS,
                 vd = xd[e], vu = xu[e], vf = fr[e];
         T sum, q;
         if (oc_coded) {
-          const T *t = ctab[b & 127u];
-          const Quad<T> c0 = *reinterpret_cast<const Quad<T> *>(t);
-          const Quad<T> c1 = *reinterpret_cast<const Quad<T> *>(t + 4);
-          sum = c0.x * vn + c0.y * vs + c0.z * ve + c0.w * vw +
-                c1.x * vd + c1.y * vu;
-          q = div_by_recip(KEEP ? vf + sum : vf + T(0) * sum, c1.z, c1.w);
+          const auto &t = ctab[b & 127u];
+          sum = t.c[0] * vn + t.c[1] * vs + t.c[2] * ve + t.c[3] * vw +
+                t.c[4] * vd + t.c[5] * vu;
+          q = t.divide(KEEP ? vf + sum : vf + T(0) * sum);
         } else {
           const int p = (int)(row + e);
           Couplings<T> cp{};
@@ -352,8 +366,8 @@ template <typename T>
 StreamShape stream_shape(const Dims &d, int resident_ctas) {
   constexpr int J = StreamCfg<T>::J;
   StreamShape sh{};
-  // entries of the longer half, rounded to the four a lane reads at once
-  // (16 bytes of float, 32 of double)
+  // entries of the longer half, rounded up to a box row of whole 16-byte
+  // pieces (16 bytes of four floats, 32 of four doubles)
   const int hx = (d.nx + 1) / 2;
   sh.bw = (hx + 3) & ~3;
   sh.bwc = (hx + 15) & ~15;

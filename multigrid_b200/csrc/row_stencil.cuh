@@ -4,6 +4,9 @@
 // a product with A reads only the vector's neighbours.
 #pragma once
 
+#include <math.h>
+#include <string.h>
+
 #include "pmg_common.cuh"
 
 namespace pmg {
@@ -145,20 +148,91 @@ private:
   }
 };
 
-// s / c from y, the reciprocal of c rounded to nearest: two residual
+// ---- division by a divisor that is divided by many times --------------------
+// s / c, the bits of the IEEE divide, from y = recip_of(c): two residual
 // corrections of the product s y. The first leaves q within an ulp of the
 // quotient, so the second gives it correctly rounded (Markstein, IBM J. Res.
-// Dev. 34, 1990), the bits of the divide, in five dependent operations (a
-// double divide is ~110 cycles, these ~40).
-__device__ __forceinline__ double div_by_recip(double s, double c, double y) {
-  double q = s * y;
-  q = __fma_rn(__fma_rn(-q, c, s), y, q);
-  return __fma_rn(__fma_rn(-q, c, s), y, q);
+// Dev. 34, 1990): five dependent operations (a double divide is ~110 cycles,
+// these ~40). That needs y correctly rounded, s - q c exact and the quotient
+// normal, which holds where c_min <= c <= c_max and q_min <= |s y| <= q_max:
+// then |s| lies between 2^-100 and 2^126 (2^-700 and 2^700 in double), and
+// s - q c, a multiple of 2^-47 (2^-105) of s, does not underflow. Everything
+// else takes the divide: infinities, NaN, tiny and huge numerators and
+// divisors out of range (their reciprocal is NaN here). A zero numerator,
+// frequent on a zero-started level, does not: the residual is taken negated,
+// q c - s, so that the zero keeps its sign. The range test is one integer
+// subtraction and comparison (of the upper half of a double).
+template <typename T> struct DivRange;
+template <> struct DivRange<float> {
+  static constexpr float c_min = 0x1p-30f, c_max = 0x1p40f;
+  static constexpr float q_min = 0x1p-70f, q_max = 0x1p86f;
+  // twice the bits of the sizes
+  static constexpr unsigned key_min = (127u - 70u) << 24,
+                            key_max = (127u + 86u) << 24;
+};
+template <> struct DivRange<double> {
+  static constexpr double c_min = 0x1p-200, c_max = 0x1p200;
+  static constexpr double q_min = 0x1p-500, q_max = 0x1p500;
+  static constexpr unsigned key_min = (1023u - 500u) << 21,
+                            key_max = (1023u + 500u) << 21;
+};
+template <typename T> __host__ __device__ __forceinline__ T recip_of(T c) {
+  using R = DivRange<T>;
+  return c >= R::c_min && c <= R::c_max ? T(1) / c : T(NAN);
 }
-__device__ __forceinline__ float div_by_recip(float s, float c, float y) {
-  float q = s * y;
-  q = __fmaf_rn(__fmaf_rn(-q, c, s), y, q);
-  return __fmaf_rn(__fmaf_rn(-q, c, s), y, q);
+__host__ __device__ __forceinline__ unsigned size_key(float v) {
+  unsigned u;
+  memcpy(&u, &v, sizeof(u));
+  return 2u * u;
+}
+__host__ __device__ __forceinline__ unsigned size_key(double v) {
+  unsigned long long u;
+  memcpy(&u, &v, sizeof(u));
+  return 2u * (unsigned)(u >> 32);
+}
+template <typename T>
+__host__ __device__ __forceinline__ T div_by_recip(T s, T c, T y) {
+  using R = DivRange<T>;
+  const T q0 = s * y;
+  T q = fma(-fma(q0, c, -s), y, q0);
+  q = fma(-fma(q, c, -s), y, q);
+  const bool outside = size_key(q0) - R::key_min > R::key_max - R::key_min;
+  const bool zero = (s == T(0)) & (q0 == T(0));
+  if (__builtin_expect(outside & !zero, 0))
+    q = s / c;
+  return q;
+}
+
+// s / c in float, the bits of the IEEE divide for every s and c without a
+// test: the double product of s with 1 / c held as hi + lo, rounded to float.
+// hi is 1 / c rounded towards zero and lo the rest, of the same sign (never
+// zero, so that an infinite s stays one and a zero keeps its sign). The fused
+// sum is s / c rounded once to double up to 2^-104 of it. A quotient that is
+// a float, or lies midway between two (only where those are subnormal), is a
+// double with room to spare and comes out exactly; any other quotient of two
+// 24-bit significands is at least 2^-49 of itself away from every such value,
+// so both roundings end at the same float.
+struct RecipPair {
+  double hi, lo;
+};
+__host__ __device__ __forceinline__ RecipPair recip_pair(float c) {
+  const double d = c;
+  double hi = 1.0 / d;
+  if (!(hi - hi == 0.0) || hi == 0.0) // c is zero, infinite or NaN
+    return RecipPair{hi, hi};
+  double rest = fma(-d, hi, 1.0); // exact
+  if (rest < 0.0) { // hi was rounded away from zero: the next towards it
+    unsigned long long u;
+    memcpy(&u, &hi, sizeof(u));
+    --u;
+    memcpy(&hi, &u, sizeof(hi));
+    rest = fma(-d, hi, 1.0);
+  }
+  return RecipPair{hi, rest == 0.0 ? hi * 0x1p-200 : rest * hi};
+}
+__host__ __device__ __forceinline__ float div_by_pair(float s, RecipPair r) {
+  const double v = s;
+  return (float)fma(v, r.hi, v * r.lo);
 }
 
 // Sum of v over the warp, the same bits in every lane.
