@@ -303,6 +303,11 @@ __global__ void atom_scatter_kernel(int natoms, const int *cid, int *fill,
 //   * exp by a table of 2^(j/64) and a degree-5 polynomial (Tang, ACM TOMS
 //     15, 1989): y = d' (-kappa 64 / ln 2) = m + f, the product in two parts
 //     so that f keeps its last bits, exp = 2^(m/64) e^(f ln 2 / 64).
+// That holds for normal results and a 32-bit m. The host bounds the arguments
+// by the grid's diagonal and the largest radius; beyond +-700 the kernel with
+// CHECK runs, whose threads take CUDA's exp for the four points of an atom
+// where one of them needs it (in the usual range the checks cost 6%: 129^3,
+// 3000 atoms, 80 registers in place of 64).
 // The block's eight warps take the same points and every eighth atom each;
 // their sums are added in warp order (deterministic; without that split a
 // 65^3 grid has too few points to fill the GPU). Every face point belongs to
@@ -324,6 +329,11 @@ struct DhParams {
   double khi, klo; // -kappa 64 / ln 2 = khi + klo
 };
 
+// exp(-kappa (d - r)) from the squared distance, for any argument
+__device__ __noinline__ double dh_exp(double kappa, double d2, double r) {
+  return exp(-kappa * (sqrt(d2) - r));
+}
+
 // the plain sum at one point (where the fast one met a zero distance)
 __device__ double dh_plain(const double *atoms, int natoms, const DhParams &b,
                            long i0, long i1, long i2) {
@@ -339,6 +349,7 @@ __device__ double dh_plain(const double *atoms, int natoms, const DhParams &b,
   return acc;
 }
 
+template <bool CHECK>
 __global__ void __launch_bounds__(32 * kDhWarps)
     boundary_kernel(const double *__restrict__ atoms, int natoms, DhParams b,
                     double *__restrict__ x0) {
@@ -396,6 +407,8 @@ __global__ void __launch_bounds__(32 * kDhWarps)
       const double da = xa - at[ax], dr = xr - at[row_ax];
       const double s = fma(da, da, dr * dr), pos = at[run_ax];
       const double rad = at[3], fac = at[4];
+      double w[kDhPoints], inv[kDhPoints];
+      bool out = false;
 #pragma unroll
       for (int q = 0; q < kDhPoints; ++q) {
         const double dc = xc[q] - pos;
@@ -414,13 +427,28 @@ __global__ void __launch_bounds__(32 * kDhWarps)
         p = fma(f, p, kDhTerm[3]);
         p = fma(f, p, kDhTerm[2]);
         p = f * fma(f, p, kDhTerm[1]);
-        double w = table[m & 63];
-        w = fma(w, p, w);
-        const int k = min(max(m >> 6, -1021), 1022);
-        w = __hiloint2double(__double2hiint(w) + (k << 20),
-                             __double2loint(w));
-        acc[q] = fma(fac * w, y, acc[q]);
+        double v = table[m & 63];
+        v = fma(v, p, v);
+        const int k = m >> 6;
+        w[q] = __hiloint2double(__double2hiint(v) + (k << 20),
+                                __double2loint(v));
+        inv[q] = y;
+        // v >= 2^-1: a normal result for k in [-1021, 1023]; the upper half
+        // of the addend, with m's sign, where m has 32 bits
+        if constexpr (CHECK)
+          out |= (unsigned)(k + 1021) > 2044u ||
+                 __double2hiint(big) != 0x43380000 + (m >> 31);
       }
+      if (CHECK && out) {
+#pragma unroll
+        for (int q = 0; q < kDhPoints; ++q) {
+          const double dc = xc[q] - pos;
+          w[q] = dh_exp(b.kappa, fma(dc, dc, s), rad);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kDhPoints; ++q)
+        acc[q] = fma(fac * w[q], inv[q], acc[q]);
     }
   }
 #pragma unroll
@@ -639,8 +667,17 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
     b.klo = (double)(k - b.khi);
     const long threads =
         (2L * n + 4L * (n - 2)) * ((n + kDhPoints - 1) / kDhPoints);
-    boundary_kernel<<<(unsigned)((threads + 31) / 32), 32 * kDhWarps, 0,
-                      st>>>(d_atoms, natoms, b, x0);
+    double rmax = 0.0;
+    for (int a = 0; a < natoms; ++a)
+      rmax = std::max(rmax, atoms_host[5 * a + 3]);
+    const double reach = std::max(2.0 * h * (n - 1), rmax); // over sqrt(3)
+    const unsigned blocks = (unsigned)((threads + 31) / 32);
+    if (p.kappa * reach <= 700.0)
+      boundary_kernel<false>
+          <<<blocks, 32 * kDhWarps, 0, st>>>(d_atoms, natoms, b, x0);
+    else
+      boundary_kernel<true>
+          <<<blocks, 32 * kDhWarps, 0, st>>>(d_atoms, natoms, b, x0);
     PMG_LAUNCH_CHECK();
   }
   return PMG_OK;
