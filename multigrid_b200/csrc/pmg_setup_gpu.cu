@@ -25,6 +25,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <limits.h>
 #include <cmath>
 #include <vector>
 
@@ -107,21 +108,21 @@ __device__ __forceinline__ void mark_sphere(int n, double h,
 __global__ void __launch_bounds__(kSetupThreads)
     mark_spheres_kernel(int n, double h, SphereSets sets) {
   const int lane = threadIdx.x & 31;
-  const int warps = (int)(gridDim.x * blockDim.x) >> 5;
-  int count[3];
+  const unsigned warps = (gridDim.x * blockDim.x) >> 5;
+  unsigned count[3]; // (their sum may pass 2^31)
 #pragma unroll
   for (int t = 0; t < 3; ++t)
     count[t] =
         sets.set[t].count_dev ? *sets.set[t].count_dev : sets.set[t].count;
-  for (int g = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  for (unsigned g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
        g < count[0] + count[1] + count[2]; g += warps) {
     if (g < count[0])
-      mark_sphere(n, h, sets.set[0], sets.axis, g, lane);
+      mark_sphere(n, h, sets.set[0], sets.axis, (int)g, lane);
     else if (g < count[0] + count[1])
-      mark_sphere(n, h, sets.set[1], sets.axis, g - count[0], lane);
+      mark_sphere(n, h, sets.set[1], sets.axis, (int)(g - count[0]), lane);
     else
-      mark_sphere(n, h, sets.set[2], sets.axis, g - count[0] - count[1],
-                  lane);
+      mark_sphere(n, h, sets.set[2], sets.axis,
+                  (int)(g - count[0] - count[1]), lane);
   }
 }
 unsigned mark_blocks(const SphereSets &s) {
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(kSetupThreads)
       }
   if (!free)
     return;
-  const int slot = atomicAdd(kept, 1);
+  const size_t slot = (size_t)atomicAdd(kept, 1); // (3 slot may pass 2^31)
   centres[3 * slot + 0] = pc[0];
   centres[3 * slot + 1] = pc[1];
   centres[3 * slot + 2] = pc[2];
@@ -510,6 +511,11 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
     set_last_message("setup_fine_device: bad argument");
     return PMG_ERR_ARG;
   }
+  const bool probe = ph->probe_radius > 0;
+  if (probe && (long)natoms * kProbePoints > INT_MAX) {
+    set_last_message("setup_fine_device: more than 2^31 probe positions");
+    return PMG_ERR_ARG;
+  }
   for (int a = 0; a < natoms; ++a) {
     for (int d = 0; d < 3; ++d) {
       const double x = atoms_host[5 * a + d];
@@ -527,7 +533,6 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
   const Physics p = physics(*ph);
   const double h2 = h * h;
   const double v_out = p.eps_out / h2, v_in = p.eps_in / h2;
-  const bool probe = ph->probe_radius > 0;
   Scratch sc(st);
   double *d_atoms = nullptr;
   unsigned char *inside = nullptr, *sas = nullptr, *carved = nullptr,

@@ -1,4 +1,6 @@
 """The GPU set-up outside the usual ranges, against the host set-up."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -10,8 +12,28 @@ if not torch.cuda.is_available():  # pragma: no cover
     pytest.skip("no CUDA device", allow_module_level=True)
 
 from multigrid_b200.molecule import DEFAULT_PHYSICS  # noqa: E402
-from multigrid_b200.problem import kappa  # noqa: E402
-from test_gpu_boundary import both  # noqa: E402
+from multigrid_b200 import _lib  # noqa: E402
+from multigrid_b200.problem import (kappa, physics_struct,  # noqa: E402
+                                    setup_fine)
+
+KEYS = ("oC", "oE", "oN", "uC", "f", "x0")
+
+
+def setup_on_gpu(n, h, atoms, physics):
+    out = {k: torch.full((n ** 3,), 7.0, dtype=torch.float64, device="cuda")
+           for k in KEYS}
+    atoms = np.ascontiguousarray(atoms, dtype=np.float64)
+    _lib.check("pmg_setup_fine_d", _lib.lib.pmg_setup_fine_d(
+        n, h, atoms.ctypes.data_as(_lib.PD), len(atoms),
+        ctypes.byref(physics_struct(physics)),
+        *[ctypes.c_void_p(out[k].data_ptr()) for k in KEYS], None))
+    torch.cuda.synchronize()
+    return {k: out[k].cpu().numpy() for k in KEYS}
+
+
+def both(n, h, atoms, physics):
+    return setup_on_gpu(n, h, atoms, physics), setup_fine(n, h, atoms,
+                                                          physics)
 
 
 def salty(salt):
@@ -65,3 +87,31 @@ def test_boundary_beyond_the_largest_double():
     assert np.array_equal(np.isinf(d), big)
     fine = ~big
     assert (np.abs(d - x0)[fine] <= 1e-12 * x0[fine]).all()
+
+
+def test_more_than_2_31_coordinates_of_kept_probe_centres():
+    """7.5 million atoms that do not touch keep all their 96 probe centres:
+    723 million rows of three coordinates. The masks at the few grid points
+    depend on the atoms near them alone, which the host sets up."""
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 40 GB of device memory")
+    n, h, per_axis = 9, 200.0, 196
+    g = (np.arange(per_axis) + 0.5) * (h * (n - 1) / per_axis)
+    physics = dict(DEFAULT_PHYSICS)
+    atoms = np.empty((per_axis ** 3, 5))
+    atoms[:, :3] = np.stack(np.meshgrid(g, g, g, indexing="ij"),
+                            -1).reshape(-1, 3)
+    atoms[:, 3] = 1.5
+    atoms[:, 4] = 0.0
+    assert len(atoms) * 96 * 3 > 2 ** 31
+    assert g[1] - g[0] > 2 * (1.5 + physics["probe_radius"])
+    # faces lie half a spacing from the points along one axis
+    off = np.abs(atoms[:, :3] / (h / 2) - np.rint(atoms[:, :3] / (h / 2)))
+    near = atoms[(off * (h / 2) < 6.0).all(axis=1)]
+    assert 1000 < len(near) < 50000
+    out = setup_on_gpu(n, h, atoms, physics)
+    host = setup_fine(n, h, near, physics)
+    for k in ("oC", "oE", "oN", "uC"):
+        want = host[k].ravel()
+        assert len(np.unique(want)) > 1, k
+        assert np.array_equal(out[k], want), k
