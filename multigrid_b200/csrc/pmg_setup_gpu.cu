@@ -52,10 +52,11 @@ struct SphereSets {
   int axis; // centres shifted by -h/2 along this axis (-1: no)
 };
 
-// The points of sphere q of a set, by one warp.
+// The points of sphere q of a set: part `part` of `parts`, by one warp.
 __device__ __forceinline__ void mark_sphere(int n, double h,
                                             const SphereSet &set, int axis,
-                                            int q, int lane) {
+                                            int q, int part, int parts,
+                                            int lane) {
   const double *row = set.centers + (size_t)q * set.stride;
   const double hx = 0.5 * h;
   const double c[3] = {axis == 0 ? row[0] - hx : row[0],
@@ -71,7 +72,7 @@ __device__ __forceinline__ void mark_sphere(int n, double h,
   const int w0 = hi0 - lo0 + 1, w1 = bhi1 - blo1 + 1;
   if (w0 <= 0 || w1 <= 0)
     return;
-  for (int t = lane; t < w0 * w1; t += 32) {
+  for (int t = lane + 32 * part; t < w0 * w1; t += 32 * parts) {
     const int i0 = lo0 + t / w1, i1 = blo1 + t % w1;
     if (i0 < 0 || i1 < 0 || i0 >= n || i1 >= n)
       continue;
@@ -104,7 +105,11 @@ __device__ __forceinline__ void mark_sphere(int n, double h,
 // the spheres. A block per sphere, with the probe positions that are not free
 // among them, spent its time starting blocks (3000 atoms, 129^3: 850 -> 216 us
 // for all marks, with the three sets of an axis in one launch; a warp per
-// sphere with the unfree ones skipped, 272 us).
+// sphere with the unfree ones skipped, 272 us). Where the spheres are fewer
+// than the grid's warps, each is split over as many warps as there are for it:
+// a few large spheres (fine grids) otherwise leave most of the GPU idle (12
+// atoms, 129^3 points 0.05 A apart: whole set-up 33 ms with a warp per sphere,
+// 6.3 with a block per sphere, 1.3 so).
 __global__ void __launch_bounds__(kSetupThreads)
     mark_spheres_kernel(int n, double h, SphereSets sets) {
   const int lane = threadIdx.x & 31;
@@ -114,21 +119,29 @@ __global__ void __launch_bounds__(kSetupThreads)
   for (int t = 0; t < 3; ++t)
     count[t] =
         sets.set[t].count_dev ? *sets.set[t].count_dev : sets.set[t].count;
-  for (unsigned g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-       g < count[0] + count[1] + count[2]; g += warps) {
+  const unsigned total = count[0] + count[1] + count[2];
+  const unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const unsigned parts = total < warps ? warps / total : 1; // (total > 0)
+  const unsigned part = w % parts;
+  for (unsigned g = w / parts; g < total; g += warps / parts) {
     if (g < count[0])
-      mark_sphere(n, h, sets.set[0], sets.axis, (int)g, lane);
+      mark_sphere(n, h, sets.set[0], sets.axis, (int)g, part, parts, lane);
     else if (g < count[0] + count[1])
-      mark_sphere(n, h, sets.set[1], sets.axis, (int)(g - count[0]), lane);
+      mark_sphere(n, h, sets.set[1], sets.axis, (int)(g - count[0]), part,
+                  parts, lane);
     else
       mark_sphere(n, h, sets.set[2], sets.axis,
-                  (int)(g - count[0] - count[1]), lane);
+                  (int)(g - count[0] - count[1]), part, parts, lane);
   }
 }
-unsigned mark_blocks(const SphereSets &s) {
-  const long q = (long)s.set[0].count + s.set[1].count + s.set[2].count;
-  const long b = (q * 32 + kSetupThreads - 1) / kSetupThreads;
-  return (unsigned)std::min(b, 148L * 8);
+// Blocks for the sets, whose radii are at most rmax: a warp per 32 columns of
+// every sphere, up to a grid that fills the GPU once.
+unsigned mark_blocks(const SphereSets &s, int n, double h, double rmax) {
+  const double q = (double)s.set[0].count + s.set[1].count + s.set[2].count;
+  const double side = std::min(2.0 * rmax / h + 2.0, (double)n);
+  const double warps = q * std::ceil(side * side / 32.0);
+  return (unsigned)std::min(std::ceil(warps * 32.0 / kSetupThreads),
+                            148.0 * 8);
 }
 
 __global__ void face_from_masks_kernel(long count, const unsigned char *inside,
@@ -529,6 +542,9 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
       return PMG_ERR_ARG;
     }
   }
+  double rmax = 0.0;
+  for (int a = 0; a < natoms; ++a)
+    rmax = std::max(rmax, atoms_host[5 * a + 3]);
   const long n3 = (long)n * n * n;
   const Physics p = physics(*ph);
   const double h2 = h * h;
@@ -564,10 +580,7 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
     // cell list of the atoms, built on the stream: edge >= the largest
     // inflated radius, at most 64 cells per axis of the grid's extent
     const double extent = h * (n - 1);
-    double cell = 0;
-    for (int a = 0; a < natoms; ++a)
-      cell = std::max(cell, atoms_host[5 * a + 3]);
-    cell = std::max(cell + ph->probe_radius, extent / 63);
+    const double cell = std::max(rmax + ph->probe_radius, extent / 63);
     const int dim = (int)(extent / cell) + 1;
     const int ncells = dim * dim * dim;
     int *d_cid = nullptr, *d_count = nullptr, *d_cstart = nullptr,
@@ -616,7 +629,9 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
         m.set[2] = SphereSet{centres,          3,         np, nullptr,
                              ph->probe_radius, kept, carved};
       }
-      mark_spheres_kernel<<<mark_blocks(m), kSetupThreads, 0, st>>>(n, h, m);
+      const unsigned blocks = mark_blocks(
+          m, n, h, probe ? rmax + ph->probe_radius : rmax);
+      mark_spheres_kernel<<<blocks, kSetupThreads, 0, st>>>(n, h, m);
     }
     face_from_masks_kernel<<<grid_for(n3), kSetupThreads, 0, st>>>(
         n3, inside, probe && natoms > 0 ? sas : nullptr, carved, v_in, v_out,
@@ -631,7 +646,8 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
     m.axis = -1;
     m.set[0] = SphereSet{d_atoms, 5, natoms, d_atoms + 3, ph->ion_radius,
                          nullptr, ion};
-    mark_spheres_kernel<<<mark_blocks(m), kSetupThreads, 0, st>>>(n, h, m);
+    mark_spheres_kernel<<<mark_blocks(m, n, h, rmax + ph->ion_radius),
+                          kSetupThreads, 0, st>>>(n, h, m);
   }
   centre_kernel<<<grid_for(n3), kSetupThreads, 0, st>>>(
       n, uC, oN, oE, ion, p.kappa * p.kappa * p.eps_out, oC);
@@ -672,9 +688,6 @@ int setup_fine_device(int n, double h, const double *atoms_host, int natoms,
     b.klo = (double)(k - b.khi);
     const long threads =
         (2L * n + 4L * (n - 2)) * ((n + kDhPoints - 1) / kDhPoints);
-    double rmax = 0.0;
-    for (int a = 0; a < natoms; ++a)
-      rmax = std::max(rmax, atoms_host[5 * a + 3]);
     const double reach = std::max(2.0 * h * (n - 1), rmax); // over sqrt(3)
     const unsigned blocks = (unsigned)((threads + 31) / 32);
     if (p.kappa * reach <= 700.0)

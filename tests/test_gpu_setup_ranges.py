@@ -115,3 +115,19 @@ def test_more_than_2_31_coordinates_of_kept_probe_centres():
         want = host[k].ravel()
         assert len(np.unique(want)) > 1, k
         assert np.array_equal(out[k], want), k
+
+
+# one sphere (every warp a part of it), a few, and as many as there are warps
+# or more; spheres that reach past the grid, and of one column
+@pytest.mark.parametrize("n,h,count,radius", [
+    (33, 0.1, 1, 5.0), (33, 0.1, 1, 0.0), (40, 0.1, 12, 1.8),
+    (65, 0.05, 3, 1.0), (33, 0.3, 150, 0.2), (33, 1.0, 400, 1.5)])
+@pytest.mark.parametrize("probe", [0.0, 1.4])
+def test_marks_of_few_and_many_spheres(n, h, count, radius, probe):
+    rng = np.random.default_rng(count + n)
+    atoms = np.column_stack([rng.uniform(0.0, (n - 1) * h, (count, 3)),
+                             np.full(count, radius),
+                             rng.normal(0, 0.5, count)])
+    dev, host = both(n, h, atoms, dict(DEFAULT_PHYSICS, probe_radius=probe))
+    for k in ("oC", "oE", "oN", "uC", "f"):
+        assert np.array_equal(dev[k], host[k].ravel()), k
