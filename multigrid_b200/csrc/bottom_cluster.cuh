@@ -123,77 +123,95 @@ __device__ __forceinline__ SplitPoint<ROW, PLANE> split_point(int i, int j,
 // when the hierarchy is built. The CG it replaces there runs 11 to 20
 // iterations of ~1500 cycles to a residual reduction of 1e-4 on 27 unknowns
 // (14 of the kernel's 41 us), and more on 125; the product takes ~1000 cycles
-// and solves to rounding. The inverse costs 19 us per build (27 unknowns).
+// and solves to rounding.
 // In-place Gauss-Jordan without pivoting (the operator is symmetric positive
 // definite; *ok = 0 where a pivot is not positive, and the CG runs): 32 x 32
 // threads, each with the elements (i, j), i = ti mod 32, j = tj mod 32, in
 // registers (one of them for 27 unknowns); each step passes one row and one
-// column through shared memory.
+// column through shared memory. A build waits for it, so a step is one
+// barrier, one multiply-add per element and the row and the column set by the
+// threads that hold them (two barriers and a choice of both in every element,
+// and four integer divisions each at the start: 252 us for 125 unknowns, 19.5
+// for 27; so 85 and 16.5).
 constexpr int kInvMax = 125;
 __global__ void __launch_bounds__(1024)
-    level1_inverse_kernel(Dims d, Op14<double> A, double *__restrict__ inv,
-                          int *__restrict__ ok) {
-  __shared__ double rowp[128], colp[128];
+    level1_inverse_kernel(Dims d, const __grid_constant__ Op14<double> A,
+                          double *__restrict__ inv, int *__restrict__ ok) {
+  __shared__ double rowp[2][128], colp[2][128], pivp[2]; // 1 / pivot
   const int mx = d.nx - 2, my = d.ny - 2, m = mx * my * (d.nz - 2);
   const int ti = threadIdx.x & 31, tj = threadIdx.x >> 5;
-  double v[4][4];
+  // the points of unknown 32 a + t: coordinates and place, -2 past the last
+  auto point = [&](int q, int &x, int &y, int &z) {
+    const int rq = q / mx;
+    z = q < m ? rq / my : -2;
+    x = q - rq * mx;
+    y = rq - z * my;
+  };
+  int ix[4], iy[4], iz[4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
+    point(ti + 32 * a, ix[a], iy[a], iz[a]);
+  double v[4][4];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int i = ti + 32 * a, j = tj + 32 * b;
+  for (int b = 0; b < 4; ++b) {
+    int jx, jy, jz;
+    point(tj + 32 * b, jx, jy, jz);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
       v[a][b] = 0.0;
-      if (i < m && j < m) {
-        const int ri = i / mx, rj = j / mx, iz = ri / my, jz = rj / my;
-        const int ix = i - ri * mx, iy = ri - iz * my;
-        const int ex = j - rj * mx - ix, ey = rj - jz * my - iy,
-                  ez = jz - iz;
-        const int p = d.at(ix + 2, iy + 2, iz + 2);
-        if (abs(ex) <= 1 && abs(ey) <= 1 && abs(ez) <= 1) {
-          const int s = upper_slot(ex, ey, ez);
-          v[a][b] =
-              i == j ? A.a[kOC][p]
-              : s    ? -A.a[s][p]
-                     : -A.a[upper_slot(-ex, -ey, -ez)]
-                           [p + ex + ey * d.sy() + ez * d.sz()];
-        }
+      const int ex = jx - ix[a], ey = jy - iy[a], ez = jz - iz[a];
+      if (iz[a] >= 0 && jz >= 0 && abs(ex) <= 1 && abs(ey) <= 1 &&
+          abs(ez) <= 1) {
+        const int p = d.at(ix[a] + 2, iy[a] + 2, iz[a] + 2);
+        const int s = upper_slot(ex, ey, ez);
+        v[a][b] = ex == 0 && ey == 0 && ez == 0 ? A.a[kOC][p]
+                  : s                           ? -A.a[s][p]
+                      : -A.a[upper_slot(-ex, -ey, -ez)]
+                            [p + ex + ey * d.sy() + ez * d.sz()];
       }
     }
+  }
   bool good = true;
-  for (int p = 0; p < m; ++p) {
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      if (32 * a >= m)
-        break;
-      if (ti + 32 * a == p)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          rowp[tj + 32 * b] = v[a][b];
-      if (tj + 32 * a == p)
+  for (int pb = 0; pb < 4; ++pb) { // step p = 32 pb + pl
+#pragma unroll 1
+    for (int pl = 0; pl < 32 && 32 * pb + pl < m; ++pl) {
+      double *row = rowp[pl & 1], *col = colp[pl & 1];
+      if (ti == pl)
 #pragma unroll
         for (int b = 0; b < 4; ++b)
-          colp[ti + 32 * b] = v[b][a];
-    }
-    __syncthreads();
-    const double piv = rowp[p], y = 1.0 / piv;
-    good = good && piv > 0.0;
+          row[tj + 32 * b] = v[pb][b];
+      if (tj == pl)
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      if (32 * a >= m)
-        break;
-      const int i = ti + 32 * a;
-      const double c = colp[i] * y;
+        for (int a = 0; a < 4; ++a)
+          col[ti + 32 * a] = v[a][pb];
+      if (ti == pl && tj == pl) {
+        pivp[pl & 1] = 1.0 / v[pb][pb];
+        good = good && v[pb][pb] > 0.0;
+      }
+      __syncthreads(); // (the next step's row and column go to the other half)
+      const double y = pivp[pl & 1];
+      double r[4];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        if (32 * b >= m)
+      for (int b = 0; b < 4; ++b)
+        r[b] = row[tj + 32 * b];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        if (32 * a >= m)
           break;
-        const int j = tj + 32 * b;
-        const double e = i == p ? 0.0 : v[a][b];
-        const double k = i == p ? -y : c;
-        v[a][b] = j == p ? -k : fma(-k, rowp[j], e);
+        const double c = col[ti + 32 * a] * y;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          v[a][b] = fma(-c, r[b], v[a][b]);
+        if (tj == pl)
+          v[a][pb] = -c;
+      }
+      if (ti == pl) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          v[pb][b] = tj == pl && b == pb ? y : y * r[b];
       }
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a)
