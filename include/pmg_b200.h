@@ -487,7 +487,8 @@ int pmg_setup_fine(int n, double h, const double *atoms, int natoms,
  * atoms are host rows, validated like pmg_setup_fine. oE oN uC oC and f are
  * bit-identical to pmg_setup_fine (same marking bounds and sums, charges
  * summed per grid point in atom order); x0 uses its own exponential and
- * reciprocal square root and agrees to a few ulp. */
+ * reciprocal square root and agrees to a few ulp. With a probe, at most 2^31
+ * probe positions (96 per atom) are taken. */
 int pmg_setup_fine_d(int n, double h, const double *atoms, int natoms,
                      const pmg_physics *phys, double *oC, double *oE,
                      double *oN, double *uC, double *f, double *x0,

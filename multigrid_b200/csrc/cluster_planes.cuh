@@ -26,20 +26,4 @@ __host__ __device__ inline int cg_plane_owner(int k, int nz) {
   return c;
 }
 
-// Sum of v over the CTA, in every thread (warp sums, then the warps in
-// order); sh holds 32 doubles.
-__device__ __forceinline__ double cg_block_sum(double v, double *sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0)
-    sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  const int nw = blockDim.x >> 5;
-  for (int w = 0; w < nw; ++w)
-    t += sh[w];
-  return t;
-}
-
 } // namespace pmg
